@@ -95,7 +95,7 @@ struct kami_vbd_solver {
 
     // multi-step launches (kami_vbd_step_n) and tuning
     int steps_per_launch = 8;
-    int reg_cap = 0;  // 0: fused kernel without a register cap; 120 / 168: the capped variants (C = 2 / 4); 2: packed
+    int reg_cap = 0;  // 0 (or 2): fused kernel without a register cap; 120 / 168: the capped variants (C = 2 / 4)
     int launch_mode = 0;  // KAMI_LAUNCH_*: hardware-scheduled tile grid, or persistent resident CTAs
     StepParams* d_steps = nullptr;
     int d_steps_cap = 0;
@@ -947,7 +947,26 @@ kami_status kami_vbd_step(kami_vbd_handle h, float dt, void* stream) {
     const StepParams sp = advance_clock(h, dt);
     const int steps = sp.substeps;
     kami_status st = on_stream(h, stream, [&](cudaStream_t s) -> kami_status {
-        if (h->form == KAMI_FORM_FUSED) {
+        if (h->form == KAMI_FORM_FUSED && h->tape_capacity > 0 && h->layout.K > 1) {
+            // groups of tiles on a handle with a tape (colour2): the plain step rounds differently there, and a
+            // segment recomputed from a checkpoint has to repeat the steps that led there to the bit, so
+            // these steps are recorded too, over and over into one row of scratch (the adjoint's
+            // buffers, which hold nothing between two backward calls)
+            StepParams sp1 = sp;
+            sp1.substeps = 1;
+            SdfParams no_sdf = h->sdf;
+            no_sdf.grid = nullptr;
+            TapeView row{};
+            row.dx = row.vl = h->d_gx;
+            row.q = h->d_gq;
+            row.x = h->d_gv;
+            row.v = h->d_gvl;
+            row.num_itr = h->pp.num_itr;
+            for (int k = 0; k < steps; k++)
+                KAMI_CUDA(launch_fused_record(h->dstate(), h->pp, sp1, k == steps - 1 ? h->sdf : no_sdf, row, h->layout.C,
+                                              h->warps_per_block, s, h->layout.K),
+                          "recorded step launch");
+        } else if (h->form == KAMI_FORM_FUSED) {
             KAMI_CUDA(launch_fused_step(h->dstate(), h->pp, sp, h->sdf, h->layout.C, h->schedule == KAMI_SCHEDULE_JACOBI,
                                         h->warps_per_block, s, nullptr, 1, h->reg_cap, h->layout.K, h->launch_mode),
                       "fused step launch");
@@ -1258,10 +1277,10 @@ kami_status kami_vbd_set_tuning(kami_vbd_handle h, int32_t slots_per_lane, int32
     if (register_cap != 0) {
         if (register_cap != 1 && register_cap != 2 && register_cap != 120 && register_cap != 168)
             return fail(KAMI_ERR_INVALID_ARGUMENT,
-                        "register_cap must be 0 (unchanged), 1 (none), 2 (packed x2), 120 or 168");
+                        "register_cap must be 0 (unchanged), 1 or 2 (none), 120 or 168");
         if (register_cap == 2 && (h->layout.C != 4 || h->layout.K != 1 || h->schedule != KAMI_SCHEDULE_COLOUR2))
             return fail(KAMI_ERR_UNSUPPORTED,
-                        "the packed FP32x2 variant runs the colour2 step with 4 slots per lane on single tiles");
+                        "register_cap 2 (the packed step) takes colour2 with 4 slots per lane on single tiles");
         const int cap = register_cap == 1 ? 0 : register_cap;
         if (cap != h->reg_cap) drop_graphs(h);
         h->reg_cap = cap;
@@ -1370,15 +1389,12 @@ kami_status kami_vbd_autotune(kami_vbd_handle h, float dt, int32_t trial_steps, 
     const int Fs[3] = {1, 4, 16};
     double rate_best = -1.0;
     int pick[4] = {h->layout.C, h->warps_per_block, h->steps_per_launch, h->reg_cap ? h->reg_cap : 1};
-    const bool colour2 = h->schedule == KAMI_SCHEDULE_COLOUR2;
     for (int C = 2; C <= 4 && st == KAMI_OK; C += 2) {  // both, in groups of tiles where strands need them
         // tiles per group for this C (strands longer than a tile); groups fix the CTA shape
         const int K = tiles_per_group_for(h->strand_begin.data(), h->ns, C);
         if (K == 0) continue;
-        // kernel variants: C = 2 plain or 120 registers; C = 4 plain, 168 registers or packed FP32x2
-        // (colour2, single tiles)
-        const int caps[3] = {1, C == 2 ? 120 : 168, 2};
-        for (int R = 0; R < (C == 4 && colour2 && K == 1 ? 3 : 2) && st == KAMI_OK; R++) {
+        const int caps[2] = {1, C == 2 ? 120 : 168};  // kernel variants: plain, or with the register cap
+        for (int R = 0; R < 2 && st == KAMI_OK; R++) {
         const int cap = caps[R];
         for (int W = 1; W <= (K == 1 ? 8 : 1) && st == KAMI_OK; W *= 2) {
             for (int fi = 0; fi < 3 && st == KAMI_OK; fi++) {
@@ -1412,10 +1428,10 @@ kami_status kami_vbd_autotune(kami_vbd_handle h, float dt, int32_t trial_steps, 
         }
     }
     if (st == KAMI_OK) st = kami_vbd_set_tuning(h, pick[0], pick[1], pick[2], pick[3]);
-    // the launch modes on the fastest shape (the packed variant has no persistent form)
+    // the launch modes on the fastest shape
     int mode_best = 0;
     const int modes[2] = {0, KAMI_LAUNCH_PERSISTENT};
-    for (int mi = 0; mi < (pick[3] == 2 ? 1 : 2) && st == KAMI_OK; mi++) {
+    for (int mi = 0; mi < 2 && st == KAMI_OK; mi++) {
         st = kami_vbd_set_launch_mode(h, modes[mi]);
         if (st == KAMI_OK) st = kami_vbd_set_state(h, snap, bytes, KAMI_MEMORY_DEVICE);
         if (st == KAMI_OK) st = kami_vbd_step_n(h, dt, trial_steps, nullptr, nullptr);

@@ -11,23 +11,23 @@
 //   then dx += (f - mean f) accel/s + mean f accel/(s + 3a)   (the exact inverse of a 1 1^T + s I),
 //   evaluated as dx + f isA + mean f isD with isA = accel/s, isD = accel/(s + 3a) - isA;
 //   orientation (quaternionLambdaItr, cosserat.cu:290-337) with V = -2 kk (e_i + dx_next - dx).
-// Missing neighbours enter as zero coefficients or are discarded by selects, so the iteration
-// loop has no data-dependent branches.
+// Missing neighbours enter as zero coefficients, so the iteration loop has no data-dependent branches.
+// Sums of two products are written with fmaf, so that each kernel built from this file rounds them as
+// written, whatever the compiler would contract.
 #pragma once
 #include "vbd_math.cuh"
 
 namespace kami {
 
 // PTX rsqrt.approx.ftz.f32: rsqrtf's approximation without the input scaling that the non-ftz form
-// adds for subnormal inputs.  Every input here is a normal float (or clamped to one), where the two
-// give the same result.
+// adds for subnormal inputs.  Every input here is a normal float, where the two give the same result.
 __device__ __forceinline__ float rsqrt_ftz(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
 
-__device__ __forceinline__ float sqrt_nonneg(float x) { return x * rsqrt_ftz(fmaxf(x, 1e-30f)); }
+__device__ __forceinline__ float rsqrt_nonneg(float x) { return rsqrt_ftz(fmaxf(x, 1e-30f)); }
 
 // The Hamilton product of qmul (vbd_common.cuh) as FMA chains: the same product in 16 instead of
 // 20 instructions, rounded differently.  qmul_conj_fma(l, r) = l * conj(r).
@@ -41,186 +41,186 @@ __device__ __forceinline__ float4 qmul_conj_fma(float4 l, float4 r) {
     return qmul_fma(l, make_float4(-r.x, -r.y, -r.z, r.w));
 }
 
-// One position update with folded coefficients (see the file comment).  Neighbour operands from
-// another strand (no segment in between: hn / hp false) are replaced by the vertex's own values
-// before they meet their zero coefficient, and vertices that do not move (upd false) keep dx, so a
-// non-finite strand cannot leak into the strands or padding that share its tile, as the
-// reference's flag tests guarantee.  Strands start at even tile positions, so only the previous
-// neighbour of an even slot and the next neighbour of an odd slot can belong to another strand;
-// the others are the same strand or padding (always finite), and guard_next / guard_prev say
-// which operands need the replacement (the results are the same bit for bit either way).  Padding
-// and pinned slots keep their dx through the final select: padding must stay finite, as the
-// strand before it reads it unguarded and a restored state does not rewrite padding.
-__device__ __forceinline__ float3 fused_position(float3 dx, float3 F0, float ddN, float kkN, float3 d3N, float3 dxN,
-                                                 float ddP, float kkP, float3 d3P, float3 dxP, float as_, float isA,
-                                                 float isD, bool hn, bool hp, bool upd, bool guard_next,
-                                                 bool guard_prev) {
-    if (guard_next) dxN = hn ? dxN : dx;
-    if (guard_prev) {
-        dxP = hp ? dxP : dx;
-        d3P = hp ? d3P : d3N;
-    }
-    float3 f;
-    f.x = F0.x + ddN * dxN.x + ddP * dxP.x - as_ * dx.x - kkN * d3N.x + kkP * d3P.x;
-    f.y = F0.y + ddN * dxN.y + ddP * dxP.y - as_ * dx.y - kkN * d3N.y + kkP * d3P.y;
-    f.z = F0.z + ddN * dxN.z + ddP * dxP.z - as_ * dx.z - kkN * d3N.z + kkP * d3P.z;
-    const float m = (f.x + f.y + f.z) * (1.f / 3.f);
-    const float3 n = f3(fmaf(m, isD, fmaf(f.x, isA, dx.x)), fmaf(m, isD, fmaf(f.y, isA, dx.y)),
-                        fmaf(m, isD, fmaf(f.z, isA, dx.z)));
-    return upd ? n : dx;
-}
-
-// One orientation update (quaternionLambdaItr), branch-free: pre/nxt say whether the previous /
-// next segment exists, upd whether this segment is updated at all; guard_prev / guard_next as in
-// fused_position.
-__device__ __forceinline__ float4 fused_orientation(float4 q, bool upd, bool pre, bool nxt, float3 Ve, float m2k,
-                                                    float3 dx, float3 dxN, float4 qPrev, float4 qrPrev, float4 qNext,
-                                                    float4 qr, bool guard_prev, bool guard_next) {
-    const float3 V = Ve + m2k * (dxN - dx);
-    if (guard_prev) qPrev = pre ? qPrev : q;  // operands from another strand never meet arithmetic
-    if (guard_next) qNext = nxt ? qNext : q;
-    const float4 P1 = qmul_fma(qPrev, qrPrev);
-    const float4 P2 = qmul_conj_fma(qNext, qr);
-    float s1 = dot4(q, P1) > 0.f ? 1.f : -1.f;
-    float s2 = dot4(q, P2) > 0.f ? 1.f : -1.f;
-    s1 = pre ? s1 : 0.f;
-    s2 = nxt ? s2 : 0.f;
-    const float4 b = make_float4(s1 * P1.x + s2 * P2.x, s1 * P1.y + s2 * P2.y, s1 * P1.z + s2 * P2.z,
-                                 s1 * P1.w + s2 * P2.w);
-    const float lambda = sqrt_nonneg(dot3(V, V)) + sqrt_nonneg(dot4(b, b));
-    const float3 bq = f3(b.x, b.y, b.z);
-    const float3 Pq = b.w * V + cross3(V, bq);
-    const float Pw = -dot3(V, bq);
-    const float4 R = make_float4(Pw + lambda * b.x, Pq.z + lambda * b.y, -Pq.y + lambda * b.z, -Pq.x + lambda * b.w);
-    const float4 n = scale4(rsqrt_ftz(dot4(R, R)), R);
-    return upd ? n : q;
-}
-
-// ---- packed FP32x2 form (sm_100 FFMA2 / FADD2 / FMUL2) ---------------------------------------------
-// With 4 slots per lane, slots {0, 2} and {1, 3} are each one colour, and every operand of a colour's
-// update pairs up with the same operand of the other slot of that colour.  The x2 kernel variant
-// keeps each pair in a float2 and updates both slots with one packed instruction per operation.
-struct F2x3 {
-    float2 x, y, z;
+// ---- packed FP32x2 updates (sm_100 FFMA2 / FADD2 / FMUL2) -----------------------------------------
+// A paired FP32 instruction does two operations in one issue slot; an operand may be negated, in one half
+// or both, or be one half used twice, at no cost, but exchanged halves cost a move.  So a vector keeps y and
+// z in one register pair and a quaternion (y, z) and (x, w): a scalar coefficient is a half used twice, and
+// the few products that need exchanged halves are scalar instructions.
+//
+// What bounds an iteration is the register file: three-operand FMAs on distinct registers run at 1.5
+// cycles a scheduler (3 packed), multiplications and additions at 1 (2), measured on loops of each.  That
+// sum is about 180 cycles a row of 32 slots and iteration, against 115 issue slots and 115 cycles of the FMA
+// pipe; the scalar updates before took 175 issue slots and 212 cycles.  Hence the signs of the two
+// quaternion products applied once to the result, missing neighbours kept out by the shuffle's source
+// lane, and predicated results instead of selects.  Packing two slots of a colour instead (four slots a
+// lane, or two tiles a warp) took 91 issue slots but the same register reads, and twice the registers: 101
+// us for 10,000 x 64, 20 iterations, against 89 here (99 before).
+//
+// Rounding.  On single tiles every sum below runs in the order, with the contractions, that this step's
+// trajectories have always had, so a groom moves to the same bits: an FP32 velocity is dx / h, and another
+// rounding of the iterations comes back in it 1e-5 to 1e-4 large on short strands over a few substeps.
+// That order differs between a tile of 2 and of 4 slots a lane, and in the host frame (FROM_E, Y_FIRST,
+// WZ_FIRST and the force in fused_step_body).  Groups of tiles (SHORT) take shorter sums and sqrt.approx: 10.3
+// ms instead of 11.1 for 6,000 strands of 100-300 vertices, 42 substeps of 32 iterations (10.9 before);
+// against 64 bits their positions and orientations err as before (2.7e-7 and 1.6e-6 relative).
+struct V3 {
+    float x;
+    float2 yz;
 };
-struct F2x4 {
-    float2 x, y, z, w;
+struct Q4 {
+    float2 yz, xw;
 };
+__device__ __forceinline__ float2 both(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
 __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
-__device__ __forceinline__ float2 sel2(bool cx, bool cy, float2 a, float2 b) {
-    return make_float2(cx ? a.x : b.x, cy ? a.y : b.y);
+__device__ __forceinline__ V3 v3(float3 a) { return {a.x, make_float2(a.y, a.z)}; }
+__device__ __forceinline__ float3 f3(V3 a) { return f3(a.x, a.yz.x, a.yz.y); }
+__device__ __forceinline__ Q4 q4(float4 a) { return {make_float2(a.y, a.z), make_float2(a.x, a.w)}; }
+__device__ __forceinline__ float4 f4(Q4 a) { return make_float4(a.xw.x, a.yz.x, a.yz.y, a.xw.y); }
+__device__ __forceinline__ float4 f4(V3 a) { return make_float4(a.x, a.yz.x, a.yz.y, 0.f); }
+__device__ __forceinline__ V3 shfl(V3 a, int lane) {
+    return {__shfl_sync(0xffffffffu, a.x, lane),
+            make_float2(__shfl_sync(0xffffffffu, a.yz.x, lane), __shfl_sync(0xffffffffu, a.yz.y, lane))};
 }
-__device__ __forceinline__ F2x3 sel23(bool cx, bool cy, F2x3 a, F2x3 b) {
-    return {sel2(cx, cy, a.x, b.x), sel2(cx, cy, a.y, b.y), sel2(cx, cy, a.z, b.z)};
+__device__ __forceinline__ Q4 shfl(Q4 a, int lane) {
+    return {make_float2(__shfl_sync(0xffffffffu, a.yz.x, lane), __shfl_sync(0xffffffffu, a.yz.y, lane)),
+            make_float2(__shfl_sync(0xffffffffu, a.xw.x, lane), __shfl_sync(0xffffffffu, a.xw.y, lane))};
 }
-__device__ __forceinline__ F2x4 sel24(bool cx, bool cy, F2x4 a, F2x4 b) {
-    return {sel2(cx, cy, a.x, b.x), sel2(cx, cy, a.y, b.y), sel2(cx, cy, a.z, b.z), sel2(cx, cy, a.w, b.w)};
+template <bool Y_FIRST>
+__device__ __forceinline__ float norm2(V3 a) {
+    const float t = Y_FIRST ? fmaf(a.yz.x, a.yz.x, __fmul_rn(a.x, a.x)) : fmaf(a.x, a.x, __fmul_rn(a.yz.x, a.yz.x));
+    return fmaf(a.yz.y, a.yz.y, t);
 }
-__device__ __forceinline__ F2x3 pack3(float3 a, float3 b) {
-    return {make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z)};
-}
-__device__ __forceinline__ F2x4 pack4(float4 a, float4 b) {
-    return {make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z), make_float2(a.w, b.w)};
-}
-__device__ __forceinline__ float3 lo3(F2x3 a) { return f3(a.x.x, a.y.x, a.z.x); }
-__device__ __forceinline__ float3 hi3(F2x3 a) { return f3(a.x.y, a.y.y, a.z.y); }
-__device__ __forceinline__ float4 lo4(F2x4 a) { return make_float4(a.x.x, a.y.x, a.z.x, a.w.x); }
-__device__ __forceinline__ float4 hi4(F2x4 a) { return make_float4(a.x.y, a.y.y, a.z.y, a.w.y); }
-
-// d3 = q e_x q* for a pair (d3_of, vbd_common.cuh)
-__device__ __forceinline__ F2x3 d3_of2(F2x4 q) {
-    F2x3 d;
-    d.x = sub2(fma2(q.w, q.w, mul2(q.x, q.x)), fma2(q.y, q.y, mul2(q.z, q.z)));
-    const float2 s1 = fma2(q.x, q.y, mul2(q.w, q.z));
-    d.y = add2(s1, s1);
-    const float2 s2 = fma2(q.x, q.z, mul2(neg2(q.w), q.y));
-    d.z = add2(s2, s2);
-    return d;
+__device__ __forceinline__ float norm2(Q4 a) {
+    return fmaf(a.xw.y, a.xw.y, fmaf(a.yz.y, a.yz.y, fmaf(a.xw.x, a.xw.x, __fmul_rn(a.yz.x, a.yz.x))));
 }
 
-// Hamilton product l r with the scalar last (qmul), and l conj(r) (qmul_conj), for pairs
-__device__ __forceinline__ F2x4 qmul2(F2x4 l, F2x4 r) {
-    F2x4 o;
-    o.x = fma2(l.w, r.x, fma2(r.w, l.x, fma2(l.y, r.z, neg2(mul2(r.y, l.z)))));
-    o.y = fma2(l.w, r.y, fma2(r.w, l.y, fma2(l.z, r.x, neg2(mul2(r.z, l.x)))));
-    o.z = fma2(l.w, r.z, fma2(r.w, l.z, fma2(l.x, r.y, neg2(mul2(r.x, l.y)))));
-    o.w = fma2(l.w, r.w, neg2(fma2(l.x, r.x, fma2(l.y, r.y, mul2(l.z, r.z)))));
-    return o;
+__device__ __forceinline__ float short_norm2(Q4 a) {
+    const float2 t = fma2(a.yz, a.yz, mul2(a.xw, a.xw));
+    return t.x + t.y;
 }
-__device__ __forceinline__ F2x4 qmul_conj2(F2x4 l, F2x4 r) {
-    return qmul2(l, F2x4{neg2(r.x), neg2(r.y), neg2(r.z), r.w});
-}
-__device__ __forceinline__ float2 dot42(F2x4 a, F2x4 b) {
-    return fma2(a.x, b.x, fma2(a.y, b.y, fma2(a.z, b.z, mul2(a.w, b.w))));
-}
-__device__ __forceinline__ float2 dot32(F2x3 a, F2x3 b) { return fma2(a.x, b.x, fma2(a.y, b.y, mul2(a.z, b.z))); }
-__device__ __forceinline__ float2 sqrt_nonneg2(float2 x) {
-    return make_float2(sqrt_nonneg(x.x), sqrt_nonneg(x.y));
+// PTX sqrt.approx.ftz.f32 (0 for 0 and for squares of lengths below 1e-19).
+__device__ __forceinline__ float sqrt_ftz(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
-// fused_position for a pair of same-colour slots; nkkN = -kkN, nas = -(a + s) are precomputed.
-// guard_next / guard_prev as in fused_position (even pair: previous; odd pair: next).
-__device__ __forceinline__ F2x3 fused_position2(F2x3 dx, F2x3 F0, float2 ddN, float2 nkkN, F2x3 d3N, F2x3 dxN,
-                                                float2 ddP, float2 kkP, F2x3 d3P, F2x3 dxP, float2 nas, float2 isA,
-                                                float2 isD, const bool* hn, const bool* hp, const bool* upd,
-                                                bool guard_next, bool guard_prev) {
-    if (guard_next) dxN = sel23(hn[0], hn[1], dxN, dx);
-    if (guard_prev) {
-        dxP = sel23(hp[0], hp[1], dxP, dx);
-        d3P = sel23(hp[0], hp[1], d3P, d3N);
+// l r  and  l conj(r): the products that need halves exchanged are written as scalars (an exchanged or
+// partly negated pair costs a move and a negation in every iteration)
+__device__ __forceinline__ Q4 qmul(Q4 l, Q4 r) {
+    const float lx = l.xw.x, ly = l.yz.x, lz = l.yz.y, rx = r.xw.x, ry = r.yz.x, rz = r.yz.y;
+    float2 yz = make_float2(fmaf(lz, rx, __fmul_rn(-rz, lx)), fmaf(lx, ry, __fmul_rn(-rx, ly)));
+    yz = fma2(both(r.xw.y), l.yz, yz);
+    const float2 t = mul2(both(lz), r.yz);
+    const float x = fmaf(r.xw.y, lx, fmaf(ly, rz, -t.x));
+    const float w = fmaf(lx, rx, fmaf(ly, ry, t.y));
+    return {fma2(both(l.xw.y), r.yz, yz), fma2(both(l.xw.y), r.xw, make_float2(x, -w))};
+}
+__device__ __forceinline__ Q4 qmul_conj(Q4 l, Q4 r) {
+    const float lx = l.xw.x, ly = l.yz.x, lz = l.yz.y, rx = r.xw.x, ry = r.yz.x, rz = r.yz.y;
+    float2 yz = make_float2(fmaf(-lz, rx, __fmul_rn(rz, lx)), fmaf(-lx, ry, __fmul_rn(rx, ly)));
+    yz = fma2(both(r.xw.y), l.yz, yz);
+    const float2 t = mul2(both(lz), r.yz);
+    const float x = fmaf(r.xw.y, lx, fmaf(-ly, rz, t.x));
+    const float w = fmaf(lx, rx, fmaf(ly, ry, t.y));
+    return {fma2(both(-l.xw.y), r.yz, yz), make_float2(fmaf(-l.xw.y, rx, x), fmaf(l.xw.y, r.xw.y, w))};
+}
+
+// Half the material axis, d3 / 2 = q e_x q* / 2 (d3_of, vbd_common.cuh); the position update's
+// coefficient carries the other factor of two.
+template <bool X_FIRST, bool WZ_FIRST, bool SHORT = false>
+__device__ __forceinline__ V3 half_axis(Q4 q) {
+    if (SHORT) {  // of a unit quaternion: (1/2 - y^2 - z^2, x y + w z, x z - w y)
+        const float2 t = mul2(both(q.xw.x), q.yz);
+        return {fmaf(-q.yz.y, q.yz.y, fmaf(-q.yz.x, q.yz.x, 0.5f)),
+                make_float2(fmaf(q.xw.y, q.yz.y, t.x), fmaf(-q.xw.y, q.yz.x, t.y))};
     }
-    F2x3 f;
-    f.x = fma2(kkP, d3P.x, fma2(nkkN, d3N.x, fma2(nas, dx.x, fma2(ddP, dxP.x, fma2(ddN, dxN.x, F0.x)))));
-    f.y = fma2(kkP, d3P.y, fma2(nkkN, d3N.y, fma2(nas, dx.y, fma2(ddP, dxP.y, fma2(ddN, dxN.y, F0.y)))));
-    f.z = fma2(kkP, d3P.z, fma2(nkkN, d3N.z, fma2(nas, dx.z, fma2(ddP, dxP.z, fma2(ddN, dxN.z, F0.z)))));
-    const float2 m = mul2(add2(add2(f.x, f.y), f.z), make_float2(1.f / 3.f, 1.f / 3.f));
-    F2x3 n;
-    n.x = fma2(m, isD, fma2(f.x, isA, dx.x));
-    n.y = fma2(m, isD, fma2(f.y, isA, dx.y));
-    n.z = fma2(m, isD, fma2(f.z, isA, dx.z));
-    return sel23(upd[0], upd[1], n, dx);
+
+    const float x = q.xw.x, y = q.yz.x, z = q.yz.y, w = q.xw.y;
+    const float xw = X_FIRST ? fmaf(x, x, __fmul_rn(w, w)) : fmaf(w, w, __fmul_rn(x, x));
+    const float d = 0.5f * fmaf(-z, z, fmaf(-y, y, xw));
+    if (WZ_FIRST) return {d, make_float2(fmaf(w, z, __fmul_rn(x, y)), fmaf(x, z, __fmul_rn(-w, y)))};
+    return {d, fma2(both(x), q.yz, make_float2(__fmul_rn(w, z), __fmul_rn(-w, y)))};
 }
 
-// fused_orientation for a pair of same-colour segments; guard_prev / guard_next as in fused_position.
-__device__ __forceinline__ F2x4 fused_orientation2(F2x4 q, const bool* upd, const bool* pre, const bool* nxt, F2x3 Ve,
-                                                   float2 m2k, F2x3 dx, F2x3 dxN, F2x4 qPrev, F2x4 qrPrev,
-                                                   F2x4 qNext, F2x4 qr, bool guard_prev, bool guard_next) {
-    F2x3 V;
-    V.x = fma2(m2k, sub2(dxN.x, dx.x), Ve.x);
-    V.y = fma2(m2k, sub2(dxN.y, dx.y), Ve.y);
-    V.z = fma2(m2k, sub2(dxN.z, dx.z), Ve.z);
-    if (guard_prev) qPrev = sel24(pre[0], pre[1], qPrev, q);
-    if (guard_next) qNext = sel24(nxt[0], nxt[1], qNext, q);
-    const F2x4 P1 = qmul2(qPrev, qrPrev);
-    const F2x4 P2 = qmul_conj2(qNext, qr);
-    const float2 d1 = dot42(q, P1), d2 = dot42(q, P2);
-    const float2 s1 = make_float2(pre[0] ? (d1.x > 0.f ? 1.f : -1.f) : 0.f, pre[1] ? (d1.y > 0.f ? 1.f : -1.f) : 0.f);
-    const float2 s2 = make_float2(nxt[0] ? (d2.x > 0.f ? 1.f : -1.f) : 0.f, nxt[1] ? (d2.y > 0.f ? 1.f : -1.f) : 0.f);
-    F2x4 b;
-    b.x = fma2(s1, P1.x, mul2(s2, P2.x));
-    b.y = fma2(s1, P1.y, mul2(s2, P2.y));
-    b.z = fma2(s1, P1.z, mul2(s2, P2.z));
-    b.w = fma2(s1, P1.w, mul2(s2, P2.w));
-    const float2 lambda = add2(sqrt_nonneg2(dot32(V, V)), sqrt_nonneg2(dot42(b, b)));
-    // P = V b e_x with V = (V, 0): R = (Pw + l b.x, Pq.z + l b.y, -Pq.y + l b.z, -Pq.x + l b.w),
-    // Pq = b.w V + V x bq, Pw = -V . bq
-    const float2 Pqx = fma2(b.w, V.x, sub2(mul2(V.y, b.z), mul2(b.y, V.z)));
-    const float2 Pqy = fma2(b.w, V.y, sub2(mul2(V.z, b.x), mul2(b.z, V.x)));
-    const float2 Pqz = fma2(b.w, V.z, sub2(mul2(V.x, b.y), mul2(b.x, V.y)));
-    const float2 Pw = neg2(fma2(V.x, b.x, fma2(V.y, b.y, mul2(V.z, b.z))));
-    F2x4 R;
-    R.x = fma2(lambda, b.x, Pw);
-    R.y = fma2(lambda, b.y, Pqz);
-    R.z = fma2(lambda, b.z, neg2(Pqy));
-    R.w = fma2(lambda, b.w, neg2(Pqx));
-    const float2 rr = dot42(R, R);
-    const float2 inv = make_float2(rsqrt_ftz(rr.x), rsqrt_ftz(rr.y));
-    const F2x4 n = {mul2(inv, R.x), mul2(inv, R.y), mul2(inv, R.z), mul2(inv, R.w)};
-    return sel24(upd[0], upd[1], n, q);
+// One position update with folded coefficients (see the file comment).  k2N / k2P are twice kkN / kkP
+// for the halved axes hN / hP.  use_n / use_p: whether the next / previous operands may meet arithmetic at
+// all (see fused_step_body); mov: whether the vertex moves.
+__device__ __forceinline__ void fused_position(V3& dx, V3 F0, float ddN, float k2N, V3 hN, V3 dxN, float ddP, float k2P,
+                                               V3 hP, V3 dxP, float as_, float isA, float isD, bool mov, bool use_n,
+                                               bool use_p) {
+    V3 f = F0;
+    auto add = [&](float c, V3 a) {
+        f.x = fmaf(c, a.x, f.x);
+        f.yz = fma2(both(c), a.yz, f.yz);
+    };
+    if (use_n) add(ddN, dxN);
+    if (use_p) add(ddP, dxP);
+    add(-as_, dx);
+    add(-k2N, hN);
+    if (use_p) add(k2P, hP);
+    const float m = ((f.x + f.yz.x) + f.yz.y) * (1.f / 3.f);
+    if (mov) {
+        dx.x = fmaf(m, isD, fmaf(f.x, isA, dx.x));
+        dx.yz = fma2(both(m), both(isD), fma2(f.yz, both(isA), dx.yz));
+    }
+}
+
+// One orientation update (quaternionLambdaItr).  qrP and qr are zero where the previous / next segment
+// is missing, so its product vanishes.  With the signs s1, s2 of the two products (cosserat.cu:316-335),
+// b = s1 P1 + s2 P2 = s1 (P1 + s1 s2 P2), and s1 is applied to the normalised result, which is linear
+// in b.  A sign test reads the sign bit of the negated dot product (set where the product is positive;
+// x - x gives +0, which counts as not positive).  R = V b e_x + lambda b with V = (V, 0), written out.
+// FROM_E: the components of Ve (all 3, or x and y) that hold the segment vector e instead of m2k e.
+template <bool SHORT, int FROM_E, bool Y_FIRST, bool WZ_FIRST>
+__device__ __forceinline__ void fused_orientation(Q4& q, V3& h, bool upd, V3 Ve, float m2k, V3 dx, V3 dxN, Q4 qPrev,
+                                                  Q4 qrP, Q4 qNext, Q4 qr, bool use_n, bool use_p) {
+    const V3 d = {dxN.x - dx.x, sub2(dxN.yz, dx.yz)};
+    V3 V;
+    if (FROM_E == 3)
+        V = {fmaf(m2k, Ve.x, __fmul_rn(m2k, d.x)), fma2(both(m2k), Ve.yz, mul2(both(m2k), d.yz))};
+    else if (FROM_E == 2)
+        V = {fmaf(m2k, Ve.x, __fmul_rn(m2k, d.x)),
+             make_float2(fmaf(m2k, Ve.yz.x, __fmul_rn(m2k, d.yz.x)), fmaf(m2k, d.yz.y, Ve.yz.y))};
+    else
+        V = {fmaf(m2k, d.x, Ve.x), fma2(both(m2k), d.yz, Ve.yz)};
+    Q4 P1 = qmul(qPrev, qrP), P2 = qmul_conj(qNext, qr);
+    const Q4 zero = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    if (!use_p) P1 = zero;
+    if (!use_n) P2 = zero;
+    const float2 t1 = fma2(q.yz, P1.yz, mul2(q.xw, P1.xw)), t2 = fma2(q.yz, P2.yz, mul2(q.xw, P2.xw));
+    const uint32_t g1 = __float_as_uint(-t1.x - t1.y), g2 = __float_as_uint(-t2.x - t2.y);
+    const float s12 = __uint_as_float(((g1 ^ g2) & 0x80000000u) | 0x3f800000u);
+    const Q4 b = {fma2(both(s12), P2.yz, P1.yz), fma2(both(s12), P2.xw, P1.xw)};
+    const float vv = norm2<Y_FIRST>(V), bb = SHORT ? short_norm2(b) : norm2(b);
+    const float lambda = SHORT ? sqrt_ftz(vv) + sqrt_ftz(bb)
+                               : fmaf(vv, rsqrt_nonneg(vv), __fmul_rn(bb, rsqrt_nonneg(bb)));
+    const float Vx = V.x, Vy = V.yz.x, Vz = V.yz.y, bx = b.xw.x, by = b.yz.x, bz = b.yz.y, bw = b.xw.y;
+    Q4 R;
+    if (SHORT) {
+        R = {fma2(both(Vx), b.yz, mul2(both(-bx), V.yz)), fma2(both(-Vx), b.xw, mul2(both(-Vy), b.yz))};
+        R.yz.x = fmaf(bw, Vz, R.yz.x);
+        R.yz.y = fmaf(-bw, Vy, R.yz.y);
+        R.xw.x = fmaf(-Vz, bz, R.xw.x);
+        R.xw.y = fmaf(Vz, by, R.xw.y);
+        R = {fma2(both(lambda), b.yz, R.yz), fma2(both(lambda), b.xw, R.xw)};
+    } else {
+        const float2 Pzy = make_float2(fmaf(bw, Vz, fmaf(Vx, by, __fmul_rn(-bx, Vy))),
+                                       fmaf(-bw, Vy, fmaf(-Vz, bx, __fmul_rn(bz, Vx))));
+        const float2 Pwx = make_float2(fmaf(-Vz, bz, fmaf(-Vx, bx, __fmul_rn(-Vy, by))),
+                                       fmaf(-bw, Vx, fmaf(-Vy, bz, __fmul_rn(by, Vz))));
+        R = {fma2(both(lambda), b.yz, Pzy), fma2(both(lambda), b.xw, Pwx)};
+    }
+    const float inv = rsqrt_ftz(SHORT ? short_norm2(R) : norm2(R));
+    const float2 si = both(__uint_as_float(__float_as_uint(inv) ^ (~g1 & 0x80000000u)));
+    if (upd) {
+        q.yz = mul2(si, R.yz);
+        q.xw = mul2(si, R.xw);
+    }
+    h = half_axis<false, WZ_FIRST, SHORT>(q);
 }
 
 // Values a group's warps hand across their tile boundaries (GROUPED: one CTA of K <= 8 warps per
@@ -235,56 +235,53 @@ struct GroupExchange {
     float4 down[8][XD_N];
 };
 
+// Floats of shared memory a slot takes in a fused kernel: position, velocity, last velocity, inverse
+// mass.  A host frame stages the tile's positions and velocities in the same cells before and after.
+enum : int { PARK_X = 0, PARK_V = 3, PARK_VL = 6, PARK_IM = 9, PARK_FLOATS = 10 };
+constexpr size_t park_bytes(int C, int warps) { return sizeof(float) * PARK_FLOATS * 32 * (size_t)C * warps; }
+enum : uint32_t { F_MOVES = 1u << 31 };  // in the kernels' flags: the vertex has mass
+
 // One launch runs `nsteps` consecutive steps, step j with clock and body transform steps[j] (or
-// `sp` when steps is null), keeping the tile's state in registers between them.  RECORD (colour2,
-// one step of one substep) additionally writes the step's start state and the iterates to a tape
-// for the adjoint (vbd_adjoint.cuh).  HOSTIO steps tile `tile` of a host frame (fused_frame_kernel):
-// `stage` holds the tile's positions then velocities from the host buffers of `hio`, 3 floats per
-// tile position p = lane * C + k, and the step writes its results back to the host buffers
-// through the same area, as well as to the device state.
+// `sp` when steps is null), keeping the tile's state on chip between them.  HOSTIO steps tile `frame_tile` of a host frame (fused_frame_kernel):
+// the warp's shared memory holds the tile's positions then velocities from the host buffers of `hio`, 3
+// floats per tile position p = lane * C + k, and the step writes its results back to the host buffers
+// through the same area, as well as to the device state.  Every fused kernel is launched with
+// park_bytes(C, warps) of dynamic shared memory.
 // EXPLICIT_TILE steps tile `frame_tile` (the persistent kernels' tile loop) instead of the launch's own.
-template <int C, bool JACOBI, bool RECORD, bool PAIRED = false, bool HOSTIO = false, bool GROUPED = false,
-          bool EXPLICIT_TILE = false>
+template <int C, bool JACOBI, bool HOSTIO = false, bool GROUPED = false, bool EXPLICIT_TILE = false>
 __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                TapeView tp, const StepParams* __restrict__ steps, int nsteps,
-                                                HostIO hio = HostIO{}, int64_t frame_tile = 0, float* stage = nullptr) {
-    static_assert(!GROUPED || !PAIRED, "tile groups run the plain step");
-    static_assert(!PAIRED || (C == 4 && !JACOBI && !RECORD), "the packed form is the colour2 step with 4 slots per lane");
-    static_assert(!(HOSTIO && RECORD), "recorded steps keep their state on the device");
-    static_assert(!(RECORD && JACOBI), "the tape records the colour2 schedule");
-    static_assert(C % 2 == 0, "slots per lane must be even");
+                                                const StepParams* __restrict__ steps, int nsteps,
+                                                HostIO hio = HostIO{}, int64_t frame_tile = 0) {
+    static_assert(C == 2 || C == 4, "2 or 4 slots per lane");
+    constexpr bool SHORT = GROUPED;
+    constexpr int FROM_E = SHORT ? 0 : HOSTIO ? 2 : 3;  // see fused_orientation
     const int lane = threadIdx.x & 31;
-    const int64_t tile = (HOSTIO || EXPLICIT_TILE)
-                             ? frame_tile
-                             : (RECORD ? tp.tile_begin : 0) + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int64_t tile = (HOSTIO || EXPLICIT_TILE) ? frame_tile
+                                                   : (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (tile >= st.num_tiles) return;  // uniform per warp (per CTA for groups: num_tiles is a multiple of K)
     const int64_t base = tile * (32LL * C) + lane;
-    // tile groups: neighbours across the warps of the CTA (see GroupExchange)
-    const int gw = threadIdx.x >> 5, gK = blockDim.x >> 5;
-    GroupExchange* gx = nullptr;
-    if constexpr (GROUPED) {
-        __shared__ GroupExchange group_exchange;
-        gx = &group_exchange;
-    }
-    auto up_put = [&](int slot, float4 v) {
-        if (GROUPED && lane == 31) gx->up[gw][slot] = v;
-    };
-    auto up_get = [&](int slot, float4 v) { return (GROUPED && lane == 0 && gw > 0) ? gx->up[gw - 1][slot] : v; };
-    auto down_put = [&](int slot, float4 v) {
-        if (GROUPED && lane == 0) gx->down[gw][slot] = v;
-    };
-    auto down_get = [&](int slot, float4 v) { return (GROUPED && lane == 31 && gw < gK - 1) ? gx->down[gw + 1][slot] : v; };
-    auto group_sync = [&]() {
-        if (GROUPED) __syncthreads();
-    };
-    auto f4 = [](float3 a) { return make_float4(a.x, a.y, a.z, 0.f); };
 
-    float3 x[C], v[C], vl[C], dx[C], d3[C], F0[C], Ve[C];
-    float4 q[C], qr[C];
-    float im[C], invl[C], kk[C], ddN[C], kkN[C], as_[C], isA[C], isD[C];
+    V3 dx[C], hd[C], F0[C], Ve[C];
+    Q4 q[C];
+    Q4 qr[C];
+    float ddN[C], k2N[C], as_[C], isA[C], isD[C];
     uint32_t fl[C];
-    bool mov[C];  // the vertex's position is updated (not pinned, not padding)
 
+    // The step's position, velocities and inverse mass are only needed between the iterations: they stay
+    // in this lane's cells of shared memory (PARK_FLOATS a slot), not in registers, during them.
+    extern __shared__ float kami_park[];
+    float* const warp_park = kami_park + (threadIdx.x >> 5) * (PARK_FLOATS * 32 * C);
+    auto cell = [&](int j, int k) -> float& { return warp_park[(j * C + k) * 32 + lane]; };
+    auto park3 = [&](int j, int k, float3 a) {
+        cell(j, k) = a.x;
+        cell(j + 1, k) = a.y;
+        cell(j + 2, k) = a.z;
+    };
+    auto parked3 = [&](int j, int k) { return f3(cell(j, k), cell(j + 1, k), cell(j + 2, k)); };
+
+    {
+    float3 x[C], v[C];
+    float im[C];
 #pragma unroll
     for (int k = 0; k < C; k++) {
         const int64_t g = base + 32LL * k;
@@ -292,54 +289,94 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
         x[k] = xyz(a);
         im[k] = a.w;
         v[k] = xyz(st.vel[g]);
-        vl[k] = xyz(st.vlast[g]);
-        q[k] = st.q[g];
-        qr[k] = st.qr[g];
+        q[k] = q4(st.q[g]);
         const float4 p = st.prm[g];
-        invl[k] = 1.f / p.x;
-        kk[k] = p.y * invl[k];
-        fl[k] = __float_as_uint(p.w);
-        mov[k] = im[k] != 0.f;
-        ddN[k] = (fl[k] & F_HAS_NEXT) ? kk[k] * invl[k] : 0.f;
-        kkN[k] = (fl[k] & F_HAS_NEXT) ? kk[k] : 0.f;
+        const float invl = 1.f / p.x;
+        const float kk = p.y * invl;
+        fl[k] = __float_as_uint(p.w) | (im[k] != 0.f ? F_MOVES : 0u);
+        ddN[k] = (fl[k] & F_HAS_NEXT) ? kk * invl : 0.f;
+        k2N[k] = (fl[k] & F_HAS_NEXT) ? 2.f * kk : 0.f;
+        // zero where segment k + 1 has no orientation update to take part in: the segment then adds
+        // nothing to its own update, and no other segment's update reads it
+        const float4 r = st.qr[g];
+        qr[k] = q4((fl[k] & F_HAS_NEXT_ORIENTATION) ? r : make_float4(0.f, 0.f, 0.f, 0.f));
     }
-    float* const sx = stage;
-    float* const sv = stage + 3 * 32 * C;
     if (HOSTIO && hio.x_in) {  // (no input buffers: the frame starts from the device state)
 #pragma unroll
         for (int k = 0; k < C; k++) {
             if (fl[k] & F_VALID) {  // padding slots keep their device values
                 const int o = 3 * (lane * C + k);
-                x[k] = f3(sx[o], sx[o + 1], sx[o + 2]);
-                v[k] = f3(sv[o], sv[o + 1], sv[o + 2]);
+                x[k] = f3(warp_park[o], warp_park[o + 1], warp_park[o + 2]);
+                v[k] = f3(warp_park[96 * C + o], warp_park[96 * C + o + 1], warp_park[96 * C + o + 2]);
             }
         }
-        __syncwarp();
+        __syncwarp();  // the staged input is read before its cells are reused
     }
-    const int64_t tS = tp.slots;
-    const int64_t tslot = base - (RECORD ? tp.tile_begin * 32LL * C : 0);  // this lane's slot in the tape window
-    const int64_t tbase = ((int64_t)tp.step * (tp.num_itr + 1)) * tS + tslot;  // tape row of iteration 0
-    if (RECORD) {
 #pragma unroll
-        for (int k = 0; k < C; k++) {
-            const int64_t o = (int64_t)tp.step * tS + tslot + 32LL * k;
-            tp.x[o] = make_float4(x[k].x, x[k].y, x[k].z, im[k]);
-            tp.v[o] = make_float4(v[k].x, v[k].y, v[k].z, 0.f);
-            tp.vl[o] = make_float4(vl[k].x, vl[k].y, vl[k].z, 0.f);
-        }
+    for (int k = 0; k < C; k++) {
+        const float3 vl = xyz(st.vlast[base + 32LL * k]);
+        park3(PARK_X, k, x[k]);
+        park3(PARK_V, k, v[k]);
+        park3(PARK_VL, k, vl);
+        cell(PARK_IM, k) = im[k];
     }
-    // constants of the previous lane's last segment (segment i-1 of slot 0)
-    float4 qrH = shfl_up4(qr[C - 1], 1);
-    float ddH = __shfl_up_sync(0xffffffffu, ddN[C - 1], 1);
-    float kkH = __shfl_up_sync(0xffffffffu, kkN[C - 1], 1);
-    if (GROUPED) {
-        up_put(XU_QR, qr[C - 1]);
-        up_put(XU_DK, make_float4(ddN[C - 1], kkN[C - 1], 0.f, 0.f));
-        group_sync();
-        qrH = up_get(XU_QR, qrH);
-        const float4 dk = up_get(XU_DK, make_float4(ddH, kkH, 0.f, 0.f));
-        ddH = dk.x;
-        kkH = dk.y;
+    }
+    // Neighbours across lanes: slot 0's previous slot is the previous lane's last one, slot C - 1's
+    // next slot the next lane's first one.  A lane whose neighbour is missing reads its own opposite slot
+    // instead, by the shuffle's source lane, so that another strand's values (which may not be finite) never
+    // meet arithmetic: with C = 2 that slot is in the same strand (or, in padding, finite), and its
+    // coefficients are zero.  With C = 4 it may belong to another strand too, as may the neighbours between
+    // slots 1 and 2 of a lane, so there the operands' use is predicated (use_next, use_prev).
+    const bool hp0 = fl[0] & F_HAS_PREV, hnL = fl[C - 1] & F_HAS_NEXT, nxL = fl[C - 1] & F_HAS_NEXT_ORIENTATION;
+    const int from_prev = hp0 ? (lane - 1) & 31 : lane, from_next = hnL ? (lane + 1) & 31 : lane,
+              from_next_q = nxL ? (lane + 1) & 31 : lane;
+    auto use_prev = [&](int k) { return C == 2 || (k & 1) || (fl[k] & F_HAS_PREV); };
+    auto use_next = [&](int k) { return C == 2 || !(k & 1) || (fl[k] & F_HAS_NEXT); };
+    auto use_next_q = [&](int k) { return C == 2 || !(k & 1) || (fl[k] & F_HAS_NEXT_ORIENTATION); };
+    // tile groups: neighbours across the warps of the CTA (see GroupExchange)
+    const int gw = threadIdx.x >> 5, gK = blockDim.x >> 5;
+    GroupExchange* gx = nullptr;
+    if constexpr (GROUPED) {
+        __shared__ GroupExchange group_exchange;
+        gx = &group_exchange;
+    }
+    const bool take_up = GROUPED && lane == 0 && gw > 0 && hp0, take_down = GROUPED && lane == 31 && gw < gK - 1 && hnL,
+               take_down_q = GROUPED && lane == 31 && gw < gK - 1 && nxL;
+    auto up_put = [&](int slot, float4 a) {
+        if (GROUPED && lane == 31) gx->up[gw][slot] = a;
+    };
+    auto down_put = [&](int slot, float4 a) {
+        if (GROUPED && lane == 0) gx->down[gw][slot] = a;
+    };
+    auto up_v = [&](int slot, V3 a) { return take_up ? v3(xyz(gx->up[gw - 1][slot])) : a; };
+    auto up_q = [&](int slot, Q4 a) { return take_up ? q4(gx->up[gw - 1][slot]) : a; };
+    auto down_v = [&](int slot, V3 a) { return take_down ? v3(xyz(gx->down[gw + 1][slot])) : a; };
+    auto down_q = [&](int slot, Q4 a) { return take_down_q ? q4(gx->down[gw + 1][slot]) : a; };
+    auto group_sync = [&]() {
+        if (GROUPED) __syncthreads();
+    };
+    auto upd = [&](int k) { return (fl[k] & F_HAS_NEXT) && !(fl[k] & F_FIX_ORIENTATION); };
+    auto mov = [&](int k) { return (fl[k] & F_MOVES) != 0; };
+
+    // constants of the previous lane's last segment (segment i-1 of slot 0), zero where there is none
+    Q4 qrH;
+    float ddH, k2H;
+    {
+        Q4 r = shfl(qr[C - 1], from_prev);
+        ddH = __shfl_sync(0xffffffffu, ddN[C - 1], from_prev);
+        k2H = __shfl_sync(0xffffffffu, k2N[C - 1], from_prev);
+        if (GROUPED) {
+            up_put(XU_QR, f4(qr[C - 1]));
+            up_put(XU_DK, make_float4(ddN[C - 1], k2N[C - 1], 0.f, 0.f));
+            group_sync();
+            r = up_q(XU_QR, r);
+            const V3 dk = up_v(XU_DK, V3{ddH, make_float2(k2H, 0.f)});
+            ddH = dk.x;
+            k2H = dk.yz.x;
+        }
+        qrH = q4(hp0 ? f4(r) : make_float4(0.f, 0.f, 0.f, 0.f));
+        ddH = hp0 ? ddH : 0.f;
+        k2H = hp0 ? k2H : 0.f;
     }
 
     const float accel = pp.accel_ratio;
@@ -351,260 +388,189 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
 
     for (int s = 0; s < sp.substeps; s++) {
         {
-            float3 e[C];
+            float3 x[C], e[C];
+#pragma unroll
+            for (int k = 0; k < C; k++) x[k] = parked3(PARK_X, k);
 #pragma unroll
             for (int k = 0; k < C - 1; k++) e[k] = x[k + 1] - x[k];
-            float3 xN0 = shfl_down3(x[0], 1);
+            V3 xN0 = shfl(v3(x[0]), from_next);
             if (GROUPED) {
-                down_put(XD_X, f4(x[0]));
+                down_put(XD_X, f4(v3(x[0])));
                 group_sync();
-                xN0 = xyz(down_get(XD_X, f4(xN0)));
+                xN0 = down_v(XD_X, xN0);
             }
-            e[C - 1] = xN0 - x[C - 1];
+            e[C - 1] = f3(xN0) - x[C - 1];
 #pragma unroll
             for (int k = 0; k < C; k++) e[k] = (fl[k] & F_HAS_NEXT) ? e[k] : f3(0.f, 0.f, 0.f);
-            float3 eH = shfl_up3(e[C - 1], 1);
+            V3 eH = shfl(v3(e[C - 1]), from_prev);
             if (GROUPED) {
-                up_put(XU_E, f4(e[C - 1]));
+                up_put(XU_E, f4(v3(e[C - 1])));
                 group_sync();
-                eH = xyz(up_get(XU_E, f4(eH)));
+                eH = up_v(XU_E, eH);
             }
+            const float3 e0 = hp0 ? f3(eH) : f3(0.f, 0.f, 0.f);
 #pragma unroll
             for (int k = 0; k < C; k++) {
-                float3 y;
-                vbd_predict(x[k], v[k], vl[k], im[k], pp, h, sp.last_h, sp.time, dx[k], y);
-                vl[k] = v[k];
+                float3 dx0, y;
+                const float3 v = parked3(PARK_V, k);
+                const float im = cell(PARK_IM, k);
+                vbd_predict(x[k], v, parked3(PARK_VL, k), im, pp, h, sp.last_h, sp.time, dx0, y);
+                park3(PARK_VL, k, v);
+                dx[k] = v3(dx0);
                 const float ddP = k > 0 ? ddN[k > 0 ? k - 1 : 0] : ddH;
-                const float3 eP = k > 0 ? e[k > 0 ? k - 1 : 0] : eH;
-                const float a = im[k] != 0.f ? 1.f / (im[k] * h * h) : 0.f;
-                const float sk = (ddN[k] + ddP) * (1.f + damp);
+                const float3 eP = k > 0 ? e[k > 0 ? k - 1 : 0] : e0;
+                const float a = im != 0.f ? 1.f / (im * h * h) : 0.f;
+                const float sk = __fmul_rn(ddN[k] + ddP, 1.f + damp);
                 as_[k] = a + sk;
-                isA[k] = im[k] != 0.f ? accel / sk : 0.f;
-                isD[k] = im[k] != 0.f ? accel / (sk + 3.f * a) - isA[k] : 0.f;
-                F0[k] = a * y + ddN[k] * e[k] - ddP * eP;
-                Ve[k] = (-2.f * kk[k]) * e[k];
-                d3[k] = d3_of(q[k]);
+                isA[k] = im != 0.f ? accel / sk : 0.f;
+                isD[k] = im != 0.f ? accel / fmaf(3.f, a, sk) - isA[k] : 0.f;
+                auto force = [&](float ya, float en, float ep) {
+                    const float n = __fmul_rn(ddN[k], en);  // a segment's product enters both its vertices
+                    return SHORT || k == 0 || (C == 2 && !HOSTIO) ? fmaf(-ddP, ep, fmaf(a, ya, n))
+                                            : __fsub_rn(__fadd_rn(__fmul_rn(a, ya), n), __fmul_rn(ddP, ep));
+                };
+                F0[k] = v3(f3(force(y.x, e[k].x, eP.x), force(y.y, e[k].y, eP.y), force(y.z, e[k].z, eP.z)));
+                const float3 ve = -k2N[k] * e[k];
+                Ve[k] = v3(C == 2 && k == 0 && FROM_E ? f3(e[k].x, e[k].y, FROM_E == 3 ? e[k].z : ve.z) : ve);
+                hd[k] = half_axis<true, false>(q[k]);
             }
         }
-        float4 qP = shfl_up4(q[C - 1], 1);
-        float3 d3P = shfl_up3(d3[C - 1], 1);  // the previous lane's d3_of(qP)
-        if (RECORD) {
-#pragma unroll
-            for (int k = 0; k < C; k++) {
-                tp.dx[tbase + 32LL * k] = make_float4(dx[k].x, dx[k].y, dx[k].z, 0.f);
-                tp.q[tbase + 32LL * k] = q[k];
-            }
-        }
-
-        if constexpr (PAIRED) {
-            // pairs of same-colour slots: A = {0, 2}, B = {1, 3}.  A's neighbours are B's slots
-            // (and the previous lane's slot 3 for slot 0); B's are A's (and the next lane's slot 0
-            // for slot 3).
-            F2x3 dxA = pack3(dx[0], dx[2]), dxB = pack3(dx[1], dx[3]);
-            F2x4 qA = pack4(q[0], q[2]), qB = pack4(q[1], q[3]);
-            F2x3 d3A = pack3(d3[0], d3[2]), d3B = pack3(d3[1], d3[3]);
-            const F2x3 F0A = pack3(F0[0], F0[2]), F0B = pack3(F0[1], F0[3]);
-            const F2x3 VeA = pack3(Ve[0], Ve[2]), VeB = pack3(Ve[1], Ve[3]);
-            const float2 ddNA = make_float2(ddN[0], ddN[2]), ddNB = make_float2(ddN[1], ddN[3]);
-            const float2 nkkNA = make_float2(-kkN[0], -kkN[2]), nkkNB = make_float2(-kkN[1], -kkN[3]);
-            const float2 ddPA = make_float2(ddH, ddN[1]), kkPA = make_float2(kkH, kkN[1]);
-            const float2 kkPB = make_float2(kkN[0], kkN[2]);
-            const float2 nasA = make_float2(-as_[0], -as_[2]), nasB = make_float2(-as_[1], -as_[3]);
-            const float2 isAA = make_float2(isA[0], isA[2]), isAB = make_float2(isA[1], isA[3]);
-            const float2 isDA = make_float2(isD[0], isD[2]), isDB = make_float2(isD[1], isD[3]);
-            const float2 m2kA = make_float2(-2.f * kk[0], -2.f * kk[2]), m2kB = make_float2(-2.f * kk[1], -2.f * kk[3]);
-            const F2x4 qrA = pack4(qr[0], qr[2]), qrB = pack4(qr[1], qr[3]), qrPA = pack4(qrH, qr[1]);
-            bool hnA[2], hpA[2], mvA[2], uoA[2], nxA[2], hnB[2], hpB[2], mvB[2], uoB[2], nxB[2];
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const uint32_t fa = fl[2 * j], fb = fl[2 * j + 1];
-                hnA[j] = fa & F_HAS_NEXT;
-                hpA[j] = fa & F_HAS_PREV;
-                mvA[j] = mov[2 * j];
-                uoA[j] = (fa & F_HAS_NEXT) && !(fa & F_FIX_ORIENTATION);
-                nxA[j] = fa & F_HAS_NEXT_ORIENTATION;
-                hnB[j] = fb & F_HAS_NEXT;
-                hpB[j] = fb & F_HAS_PREV;
-                mvB[j] = mov[2 * j + 1];
-                uoB[j] = (fb & F_HAS_NEXT) && !(fb & F_FIX_ORIENTATION);
-                nxB[j] = fb & F_HAS_NEXT_ORIENTATION;
-            }
-            for (int it = 0; it < pp.num_itr; it++) {
-                // positions, even slots
-                const F2x3 dxPA = pack3(shfl_up3(hi3(dxB), 1), lo3(dxB));
-                const F2x3 d3PA = pack3(shfl_up3(hi3(d3B), 1), lo3(d3B));
-                dxA = fused_position2(dxA, F0A, ddNA, nkkNA, d3A, dxB, ddPA, kkPA, d3PA, dxPA, nasA, isAA, isDA, hnA,
-                                      hpA, mvA, false, true);
-                // positions, odd slots
-                const F2x3 dxNB = pack3(hi3(dxA), shfl_down3(lo3(dxA), 1));
-                dxB = fused_position2(dxB, F0B, ddNB, nkkNB, d3B, dxNB, ddNA, kkPB, d3A, dxA, nasB, isAB, isDB, hnB, hpB,
-                                      mvB, true, false);
-                // orientations, even segments
-                const F2x4 qPA = pack4(shfl_up4(hi4(qB), 1), lo4(qB));
-                qA = fused_orientation2(qA, uoA, hpA, nxA, VeA, m2kA, dxA, dxB, qPA, qrPA, qB, qrA, true, false);
-                d3A = d3_of2(qA);
-                // orientations, odd segments
-                const F2x4 qNB = pack4(hi4(qA), shfl_down4(lo4(qA), 1));
-                qB = fused_orientation2(qB, uoB, hpB, nxB, VeB, m2kB, dxB, dxNB, qA, qrA, qNB, qrB, false, true);
-                d3B = d3_of2(qB);
-            }
-            dx[0] = lo3(dxA);
-            dx[2] = hi3(dxA);
-            dx[1] = lo3(dxB);
-            dx[3] = hi3(dxB);
-            q[0] = lo4(qA);
-            q[2] = hi4(qA);
-            q[1] = lo4(qB);
-            q[3] = hi4(qB);
-        } else {  // (braced: an unbraced discarded `else for` also dropped the loop after it)
+        auto position = [&](V3& d, int k, V3 dN, V3 dP, V3 hP) {
+            const int kp = k > 0 ? k - 1 : 0;
+            fused_position(d, F0[k], ddN[k], k2N[k], hd[k], dN, k ? ddN[kp] : ddH, k ? k2N[kp] : k2H, hP, dP, as_[k],
+                           isA[k], isD[k], mov(k), use_next(k), use_prev(k));
+        };
+        auto orientation = [&](Q4& n, V3& hn, int k, V3 dN, Q4 qP, Q4 qN) {
+            const int kp = k > 0 ? k - 1 : 0;
+            if (C == 2 && k == 0)
+                fused_orientation<SHORT, FROM_E, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qrH, qN, qr[k], use_next_q(k),
+                                               use_prev(k));
+            else if (C == 4 && (k & 1))
+                fused_orientation<SHORT, 0, !JACOBI, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qr[kp], qN, qr[k],
+                                               use_next_q(k), use_prev(k));
+            else
+                fused_orientation<SHORT, 0, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, k ? qr[kp] : qrH, qN, qr[k],
+                                                use_next_q(k), use_prev(k));
+        };
+        Q4 qP = shfl(q[C - 1], from_prev);
+        V3 hP = shfl(hd[C - 1], from_prev);  // the previous lane's half axis
         for (int it = 0; it < pp.num_itr; it++) {
+            V3 dxP = shfl(dx[C - 1], from_prev);
+            if (GROUPED) {  // the previous lane's last slot, unchanged until the odd sweeps
+                up_put(XU_DX, f4(dx[C - 1]));
+                up_put(XU_Q, f4(q[C - 1]));
+                up_put(XU_D3, f4(hd[C - 1]));
+                if (JACOBI) down_put(XD_DX, f4(dx[0]));
+                group_sync();
+                dxP = up_v(XU_DX, dxP);
+                qP = up_q(XU_Q, qP);
+                hP = up_v(XU_D3, hP);
+            }
             if (!JACOBI) {
-                float3 dxP = shfl_up3(dx[C - 1], 1);
-                if (GROUPED) {  // the previous lane's odd values, unchanged until the odd sweeps
-                    up_put(XU_DX, f4(dx[C - 1]));
-                    up_put(XU_Q, q[C - 1]);
-                    up_put(XU_D3, f4(d3[C - 1]));
-                    group_sync();
-                    dxP = xyz(up_get(XU_DX, f4(dxP)));
-                    qP = up_get(XU_Q, qP);
-                    d3P = xyz(up_get(XU_D3, f4(d3P)));
-                }
                 // positions, even slots (neighbours are odd: own registers or the previous lane)
-                {
-#pragma unroll
-                    for (int k = 0; k < C; k += 2) {
-                        const int kp = k > 0 ? k - 1 : 0;
-                        dx[k] = fused_position(dx[k], F0[k], ddN[k], kkN[k], d3[k], dx[k + 1], k ? ddN[kp] : ddH,
-                                               k ? kkN[kp] : kkH, k ? d3[kp] : d3P, k ? dx[kp] : dxP, as_[k], isA[k],
-                                               isD[k], fl[k] & F_HAS_NEXT, fl[k] & F_HAS_PREV, mov[k], false, true);
-                    }
-                }
-                // positions, odd slots
-                float3 dxN0 = shfl_down3(dx[0], 1);
-                if (GROUPED) {
-                    down_put(XD_DX, f4(dx[0]));
-                    group_sync();
-                    dxN0 = xyz(down_get(XD_DX, f4(dxN0)));
-                }
-#pragma unroll
-                for (int k = 1; k < C; k += 2) {
-                    const int kn = k + 1 < C ? k + 1 : k;
-                    dx[k] = fused_position(dx[k], F0[k], ddN[k], kkN[k], d3[k], k == C - 1 ? dxN0 : dx[kn], ddN[k - 1],
-                                           kkN[k - 1], d3[k - 1], dx[k - 1], as_[k], isA[k], isD[k],
-                                           fl[k] & F_HAS_NEXT, fl[k] & F_HAS_PREV, mov[k], true, false);
-                }
-                // orientations, even segments
 #pragma unroll
                 for (int k = 0; k < C; k += 2) {
                     const int kp = k > 0 ? k - 1 : 0;
-                    const uint32_t f = fl[k];
-                    q[k] = fused_orientation(q[k], (f & F_HAS_NEXT) && !(f & F_FIX_ORIENTATION), f & F_HAS_PREV,
-                                             f & F_HAS_NEXT_ORIENTATION, Ve[k], -2.f * kk[k], dx[k], dx[k + 1],
-                                             k ? q[kp] : qP, k ? qr[kp] : qrH, q[k + 1], qr[k], true, false);
-                    d3[k] = d3_of(q[k]);
+                    position(dx[k], k, dx[k + 1], k ? dx[kp] : dxP, k ? hd[kp] : hP);
                 }
-                // orientations, odd segments
-                float4 qN0 = shfl_down4(q[0], 1);
+                // positions, odd slots
+                V3 dxN = shfl(dx[0], from_next);
                 if (GROUPED) {
-                    down_put(XD_Q, q[0]);
+                    down_put(XD_DX, f4(dx[0]));
                     group_sync();
-                    qN0 = down_get(XD_Q, qN0);
+                    dxN = down_v(XD_DX, dxN);
+                }
+#pragma unroll
+                for (int k = 1; k < C; k += 2)
+                    position(dx[k], k, k == C - 1 ? dxN : dx[k + 1 < C ? k + 1 : k], dx[k - 1], hd[k - 1]);
+                // orientations, even segments
+#pragma unroll
+                for (int k = 0; k < C; k += 2) orientation(q[k], hd[k], k, dx[k + 1], k ? q[k > 0 ? k - 1 : 0] : qP, q[k + 1]);
+                // orientations, odd segments
+                Q4 qN = shfl(q[0], from_next_q);
+                if (GROUPED) {
+                    down_put(XD_Q, f4(q[0]));
+                    group_sync();
+                    qN = down_q(XD_Q, qN);
                 }
 #pragma unroll
                 for (int k = 1; k < C; k += 2) {
                     const int kn = k + 1 < C ? k + 1 : k;
-                    const uint32_t f = fl[k];
-                    q[k] = fused_orientation(q[k], (f & F_HAS_NEXT) && !(f & F_FIX_ORIENTATION), f & F_HAS_PREV,
-                                             f & F_HAS_NEXT_ORIENTATION, Ve[k], -2.f * kk[k], dx[k],
-                                             k == C - 1 ? dxN0 : dx[kn], q[k - 1], qr[k - 1],
-                                             k == C - 1 ? qN0 : q[kn], qr[k], false, true);
-                    d3[k] = d3_of(q[k]);
-                }
-                qP = shfl_up4(q[C - 1], 1);
-                d3P = shfl_up3(d3[C - 1], 1);
-                if (RECORD) {
-                    const int64_t row = tbase + (int64_t)(it + 1) * tS;
-#pragma unroll
-                    for (int k = 0; k < C; k++) {
-                        tp.dx[row + 32LL * k] = make_float4(dx[k].x, dx[k].y, dx[k].z, 0.f);
-                        tp.q[row + 32LL * k] = q[k];
-                    }
+                    orientation(q[k], hd[k], k, k == C - 1 ? dxN : dx[kn], q[k - 1], k == C - 1 ? qN : q[kn]);
                 }
             } else {
                 // positions, every slot from the previous sweep
-                float3 dxP = shfl_up3(dx[C - 1], 1);
-                float3 dxN0 = shfl_down3(dx[0], 1);
-                if (GROUPED) {
-                    up_put(XU_DX, f4(dx[C - 1]));
-                    up_put(XU_Q, q[C - 1]);
-                    up_put(XU_D3, f4(d3[C - 1]));
-                    down_put(XD_DX, f4(dx[0]));
-                    group_sync();
-                    dxP = xyz(up_get(XU_DX, f4(dxP)));
-                    qP = up_get(XU_Q, qP);
-                    d3P = xyz(up_get(XU_D3, f4(d3P)));
-                    dxN0 = xyz(down_get(XD_DX, f4(dxN0)));
-                }
-                float3 nd[C];
+                V3 dxN = shfl(dx[0], from_next);
+                if (GROUPED) dxN = down_v(XD_DX, dxN);
+                V3 nd[C];
 #pragma unroll
                 for (int k = 0; k < C; k++) {
                     const int kp = k > 0 ? k - 1 : 0, kn = k + 1 < C ? k + 1 : k;
-                    nd[k] = fused_position(dx[k], F0[k], ddN[k], kkN[k], d3[k], k == C - 1 ? dxN0 : dx[kn],
-                                           k ? ddN[kp] : ddH, k ? kkN[kp] : kkH, k ? d3[kp] : d3P, k ? dx[kp] : dxP,
-                                           as_[k], isA[k], isD[k], fl[k] & F_HAS_NEXT, fl[k] & F_HAS_PREV, mov[k],
-                                           (k & 1) != 0, (k & 1) == 0);
+                    nd[k] = dx[k];
+                    position(nd[k], k, k == C - 1 ? dxN : dx[kn], k ? dx[kp] : dxP, k ? hd[kp] : hP);
                 }
 #pragma unroll
                 for (int k = 0; k < C; k++) dx[k] = nd[k];
                 // orientations, every segment from the previous sweep
-                float3 dxN1 = shfl_down3(dx[0], 1);
-                float4 qN0 = shfl_down4(q[0], 1);
+                dxN = shfl(dx[0], from_next);
+                Q4 qN = shfl(q[0], from_next_q);
                 if (GROUPED) {
                     down_put(XD_DX2, f4(dx[0]));
-                    down_put(XD_Q, q[0]);
+                    down_put(XD_Q, f4(q[0]));
                     group_sync();
-                    dxN1 = xyz(down_get(XD_DX2, f4(dxN1)));
-                    qN0 = down_get(XD_Q, qN0);
+                    dxN = down_v(XD_DX2, dxN);
+                    qN = down_q(XD_Q, qN);
                 }
-                float4 nq[C];
+                Q4 nq[C];
 #pragma unroll
                 for (int k = 0; k < C; k++) {
                     const int kp = k > 0 ? k - 1 : 0, kn = k + 1 < C ? k + 1 : k;
-                    const uint32_t f = fl[k];
-                    nq[k] = fused_orientation(q[k], (f & F_HAS_NEXT) && !(f & F_FIX_ORIENTATION), f & F_HAS_PREV,
-                                              f & F_HAS_NEXT_ORIENTATION, Ve[k], -2.f * kk[k], dx[k],
-                                              k == C - 1 ? dxN1 : dx[kn], k ? q[kp] : qP, k ? qr[kp] : qrH,
-                                              k == C - 1 ? qN0 : q[kn], qr[k], (k & 1) == 0, (k & 1) != 0);
+                    nq[k] = q[k];
+                    orientation(nq[k], hd[k], k, k == C - 1 ? dxN : dx[kn], k ? q[kp] : qP, k == C - 1 ? qN : q[kn]);
                 }
 #pragma unroll
-                for (int k = 0; k < C; k++) {
-                    q[k] = nq[k];
-                    d3[k] = d3_of(q[k]);
-                }
-                qP = shfl_up4(q[C - 1], 1);
-                d3P = shfl_up3(d3[C - 1], 1);
+                for (int k = 0; k < C; k++) q[k] = nq[k];
             }
+            qP = shfl(q[C - 1], from_prev);
+            hP = shfl(hd[C - 1], from_prev);
         }
-        }  // scalar iterations
+        asm volatile("" ::: "memory");  // the parked values are read back, not kept in registers meanwhile
 #pragma unroll
-        for (int k = 0; k < C; k++) vbd_finish(x[k], v[k], dx[k], im[k], h, pp.velocity_decay);
+        for (int k = 0; k < C; k++) {
+            float3 x = parked3(PARK_X, k), v = parked3(PARK_V, k);
+            vbd_finish(x, v, f3(dx[k]), cell(PARK_IM, k), h, pp.velocity_decay);
+            park3(PARK_X, k, x);
+            park3(PARK_V, k, v);
+        }
     }
 #pragma unroll
     for (int k = 0; k < C; k++) {
-        if (sdf.grid && (fl[k] & F_VALID) && !(fl[k] & F_ROOT)) vbd_sdf(x[k], v[k], sdf, sp);
-        bad |= !finite3(x[k]) || !finite3(v[k]) || !finite4(q[k]);
+        float3 x = parked3(PARK_X, k), v = parked3(PARK_V, k);
+        if (sdf.grid && (fl[k] & F_VALID) && !(fl[k] & F_ROOT)) {
+            vbd_sdf(x, v, sdf, sp);
+            park3(PARK_X, k, x);
+            park3(PARK_V, k, v);
+        }
+        bad |= !finite3(x) || !finite3(v) || !finite4(f4(q[k]));
     }
     }  // steps
 
+    float3 x[C], v[C];
 #pragma unroll
     for (int k = 0; k < C; k++) {
         const int64_t g = base + 32LL * k;
-        st.xm[g] = make_float4(x[k].x, x[k].y, x[k].z, im[k]);
+        x[k] = parked3(PARK_X, k);
+        v[k] = parked3(PARK_V, k);
+        const float3 vl = parked3(PARK_VL, k);
+        st.xm[g] = make_float4(x[k].x, x[k].y, x[k].z, cell(PARK_IM, k));
         st.vel[g] = make_float4(v[k].x, v[k].y, v[k].z, 0.f);
-        st.vlast[g] = make_float4(vl[k].x, vl[k].y, vl[k].z, 0.f);
-        st.q[g] = q[k];
+        st.vlast[g] = make_float4(vl.x, vl.y, vl.z, 0.f);
+        st.q[g] = f4(q[k]);
     }
     if (HOSTIO && hio.x_out) {  // (no output buffers: the results stay on the device)
+        float* const sx = warp_park;
+        float* const sv = warp_park + 96 * C;
+        __syncwarp();  // every lane has read its cells
 #pragma unroll
         for (int k = 0; k < C; k++) {
             const int o = 3 * (lane * C + k);
@@ -630,17 +596,10 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(st.status, STATUS_NONFINITE);
 }
 
-template <int C, bool JACOBI, bool RECORD>
+template <int C, bool JACOBI>
 __global__ void __launch_bounds__(256) fused_step_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                         TapeView tp, const StepParams* __restrict__ steps, int nsteps) {
-    fused_step_body<C, JACOBI, RECORD>(st, pp, sp, sdf, tp, steps, nsteps);
-}
-
-// The colour2 step with 4 slots per lane in the packed FP32x2 form (the `x2` kernel variant).
-template <int C>
-__global__ void __launch_bounds__(256) fused_step_kernel_x2(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                            TapeView tp, const StepParams* __restrict__ steps, int nsteps) {
-    fused_step_body<C, false, false, true>(st, pp, sp, sdf, tp, steps, nsteps);
+                                                         const StepParams* __restrict__ steps, int nsteps) {
+    fused_step_body<C, JACOBI>(st, pp, sp, sdf, steps, nsteps);
 }
 
 // ---- host frames: one launch uploads, steps and downloads ---------------------------------------------
@@ -650,13 +609,13 @@ __global__ void __launch_bounds__(256) fused_step_kernel_x2(DeviceState st, Phys
 // over PCIe), steps the tile and writes it back (fused_step_body, HOSTIO).  The waves of tiles keep
 // the host reads of one wave apart from the host writes of the wave before, which is faster here
 // than interleaving them: SM-issued reads and writes over PCIe slow each other down.
-template <int C, bool JACOBI, bool PAIRED, bool GROUPED = false>
+template <int C, bool JACOBI, bool GROUPED = false>
 __device__ __forceinline__ void fused_frame(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf, HostIO hio) {
-    extern __shared__ float kami_frame_stage[];
+    extern __shared__ float kami_park[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
     if (t >= st.num_tiles) return;  // uniform per warp (per CTA for groups)
-    float* const stage = kami_frame_stage + w * (6 * 32 * C);
+    float* const stage = kami_park + w * (PARK_FLOATS * 32 * C);
     const int r_end = hio.x_in ? hio.run_begin[t + 1] : 0;
     for (int r = hio.run_begin[t]; r < r_end; r++) {
         const int4 run = hio.runs[r];
@@ -668,31 +627,31 @@ __device__ __forceinline__ void fused_frame(DeviceState st, PhysParams pp, StepP
         }
     }
     __syncwarp();
-    fused_step_body<C, JACOBI, false, PAIRED, true, GROUPED>(st, pp, sp, sdf, TapeView{}, nullptr, 1, hio, t, stage);
+    fused_step_body<C, JACOBI, true, GROUPED>(st, pp, sp, sdf, nullptr, 1, hio, t);
 }
-template <int C, bool JACOBI, bool PAIRED>
+template <int C, bool JACOBI>
 __global__ void __launch_bounds__(256) fused_frame_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
                                                           HostIO hio) {
-    fused_frame<C, JACOBI, PAIRED>(st, pp, sp, sdf, hio);
+    fused_frame<C, JACOBI>(st, pp, sp, sdf, hio);
 }
 template <int C, bool JACOBI>
 __global__ void __maxnreg__(120) fused_frame_kernel_r120(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
                                                         HostIO hio) {
-    fused_frame<C, JACOBI, false>(st, pp, sp, sdf, hio);
+    fused_frame<C, JACOBI>(st, pp, sp, sdf, hio);
 }
 // The same over groups of tiles: one CTA of K warps per group.
 template <int C, bool JACOBI>
 __global__ void __launch_bounds__(256) fused_frame_group_kernel(DeviceState st, PhysParams pp, StepParams sp,
                                                                 SdfParams sdf, HostIO hio) {
-    fused_frame<C, JACOBI, false, true>(st, pp, sp, sdf, hio);
+    fused_frame<C, JACOBI, true>(st, pp, sp, sdf, hio);
 }
 
 // The step with 4 slots per lane at most 168 registers per thread (a few bytes of spills): 12 instead
 // of 8 warps share an SM, which hides more of the colour sweeps' dependency latency.
 template <int C, bool JACOBI>
 __global__ void __maxnreg__(168) fused_step_kernel_r168(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                       TapeView tp, const StepParams* __restrict__ steps, int nsteps) {
-    fused_step_body<C, JACOBI, false>(st, pp, sp, sdf, tp, steps, nsteps);
+                                                       const StepParams* __restrict__ steps, int nsteps) {
+    fused_step_body<C, JACOBI>(st, pp, sp, sdf, steps, nsteps);
 }
 
 // The step over groups of K tiles (strands longer than a tile): one CTA of K warps per group, plain
@@ -700,32 +659,25 @@ __global__ void __maxnreg__(168) fused_step_kernel_r168(DeviceState st, PhysPara
 template <int C, bool JACOBI>
 __global__ void __launch_bounds__(256) fused_group_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
                                                           const StepParams* __restrict__ steps, int nsteps) {
-    fused_step_body<C, JACOBI, false, false, false, true>(st, pp, sp, sdf, TapeView{}, steps, nsteps);
+    fused_step_body<C, JACOBI, false, true>(st, pp, sp, sdf, steps, nsteps);
 }
 template <int C, bool JACOBI>
 __global__ void __maxnreg__(120) fused_group_kernel_r120(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
                                                         const StepParams* __restrict__ steps, int nsteps) {
-    fused_step_body<C, JACOBI, false, false, false, true>(st, pp, sp, sdf, TapeView{}, steps, nsteps);
+    fused_step_body<C, JACOBI, false, true>(st, pp, sp, sdf, steps, nsteps);
 }
 template <int C, bool JACOBI>
 __global__ void __maxnreg__(168) fused_group_kernel_r168(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
                                                         const StepParams* __restrict__ steps, int nsteps) {
-    fused_step_body<C, JACOBI, false, false, false, true>(st, pp, sp, sdf, TapeView{}, steps, nsteps);
-}
-
-// The recorded step (kami_vbd_step_record) over groups of tiles: one CTA of K warps per group.
-template <int C>
-__global__ void __launch_bounds__(256) fused_record_group_kernel(DeviceState st, PhysParams pp, StepParams sp,
-                                                                 SdfParams sdf, TapeView tp) {
-    fused_step_body<C, false, true, false, false, true>(st, pp, sp, sdf, tp, nullptr, 1);
+    fused_step_body<C, JACOBI, false, true>(st, pp, sp, sdf, steps, nsteps);
 }
 
 // The same step with at most 120 registers per thread, so 17 warps (instead of 16) share an SM: a
 // launch whose tile count is just above a multiple of 16 warps per SM then needs one wave less.
 template <int C, bool JACOBI>
 __global__ void __maxnreg__(120) fused_step_kernel_r120(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                       TapeView tp, const StepParams* __restrict__ steps, int nsteps) {
-    fused_step_body<C, JACOBI, false>(st, pp, sp, sdf, tp, steps, nsteps);
+                                                       const StepParams* __restrict__ steps, int nsteps) {
+    fused_step_body<C, JACOBI>(st, pp, sp, sdf, steps, nsteps);
 }
 
 // ---- persistent form ----------------------------------------------------------------------------
@@ -737,8 +689,8 @@ __device__ __forceinline__ void fused_persistent(DeviceState st, PhysParams pp, 
                                                  const StepParams* __restrict__ steps, int nsteps) {
     // only the 32-bit unit index stays live across the step body (register pressure)
     for (int u = blockIdx.x; (int64_t)u * (blockDim.x >> 5) < st.num_tiles; u += gridDim.x) {
-        fused_step_body<C, JACOBI, false, false, false, GROUPED, true>(
-            st, pp, sp, sdf, TapeView{}, steps, nsteps, HostIO{}, (int64_t)u * (blockDim.x >> 5) + (threadIdx.x >> 5));
+        fused_step_body<C, JACOBI, false, GROUPED, true>(
+            st, pp, sp, sdf, steps, nsteps, HostIO{}, (int64_t)u * (blockDim.x >> 5) + (threadIdx.x >> 5));
         if (GROUPED) __syncthreads();  // the group exchange area is reused by the next group
     }
 }

@@ -648,12 +648,12 @@ cudaError_t launch_strain_limit(float4* xm, const float4* prm, const int64_t* ro
 bool fused_supported(int C) { return C == 2 || C == 4; }
 
 namespace {
-// Launches a frame kernel: one warp per tile, 6 * 32C floats of staging per warp.
+// Launches a frame kernel: one warp per tile.
 template <typename K>
 cudaError_t launch_frame(K kernel, int C, const DeviceState& st, const PhysParams& pp, const StepParams& sp,
                          const SdfParams& sdf, const HostIO& hio, int warps_per_block, cudaStream_t s) {
-    const size_t smem = sizeof(float) * 6 * 32 * (size_t)C * warps_per_block;
-    kernel<<<blocks_for(st.num_tiles, warps_per_block), 32 * warps_per_block, smem, s>>>(st, pp, sp, sdf, hio);
+    kernel<<<blocks_for(st.num_tiles, warps_per_block), 32 * warps_per_block, park_bytes(C, warps_per_block), s>>>(
+        st, pp, sp, sdf, hio);
     return cudaGetLastError();
 }
 }  // namespace
@@ -673,23 +673,21 @@ cudaError_t launch_fused_frame(const DeviceState& st, const PhysParams& pp, cons
         return cudaErrorInvalidValue;
     }
     if (blocks_for(st.num_tiles, warps_per_block) == 0) return cudaSuccess;
-    if (reg_cap == 2 && C == 4 && !jacobi)
-        return launch_frame(fused_frame_kernel<4, false, true>, 4, st, pp, sp, sdf, hio, warps_per_block, s);
     if (reg_cap == 120 && C == 2)
         return jacobi ? launch_frame(fused_frame_kernel_r120<2, true>, 2, st, pp, sp, sdf, hio, warps_per_block, s)
                       : launch_frame(fused_frame_kernel_r120<2, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s);
     if (C == 2)
-        return jacobi ? launch_frame(fused_frame_kernel<2, true, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s)
-                      : launch_frame(fused_frame_kernel<2, false, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s);
+        return jacobi ? launch_frame(fused_frame_kernel<2, true>, 2, st, pp, sp, sdf, hio, warps_per_block, s)
+                      : launch_frame(fused_frame_kernel<2, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s);
     if (C == 4)
-        return jacobi ? launch_frame(fused_frame_kernel<4, true, false>, 4, st, pp, sp, sdf, hio, warps_per_block, s)
-                      : launch_frame(fused_frame_kernel<4, false, false>, 4, st, pp, sp, sdf, hio, warps_per_block, s);
+        return jacobi ? launch_frame(fused_frame_kernel<4, true>, 4, st, pp, sp, sdf, hio, warps_per_block, s)
+                      : launch_frame(fused_frame_kernel<4, false>, 4, st, pp, sp, sdf, hio, warps_per_block, s);
     return cudaErrorInvalidValue;
 }
 
 // Resident CTAs of `kernel` at `threads` threads on the current device (cached per device, kernel
 // and block size), times the SM count.
-static cudaError_t resident_ctas(const void* kernel, int threads, int64_t* out) {
+static cudaError_t resident_ctas(const void* kernel, int threads, size_t smem, int64_t* out) {
     static std::mutex mu;
     static std::map<std::tuple<int, const void*, int>, int64_t> cache;
     int dev = 0;
@@ -703,7 +701,7 @@ static cudaError_t resident_ctas(const void* kernel, int threads, int64_t* out) 
         return cudaSuccess;
     }
     int per_sm = 0, sms = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, 0)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     *out = cache[key] = (int64_t)std::max(1, per_sm) * sms;
     return cudaSuccess;
@@ -712,22 +710,22 @@ static cudaError_t resident_ctas(const void* kernel, int threads, int64_t* out) 
 // The persistent grid for `units` units of work: the resident CTA count, or fewer when there are
 // fewer units.  (A smaller grid that gives every CTA the same number of units was measured slower:
 // the SMs then hold unequal numbers of CTAs, and the SM with the most sets the time.)
-static cudaError_t persistent_grid(const void* kernel, int threads, int64_t units, unsigned* grid) {
+static cudaError_t persistent_grid(const void* kernel, int threads, size_t smem, int64_t units, unsigned* grid) {
     int64_t resident = 0;
-    cudaError_t e = resident_ctas(kernel, threads, &resident);
+    cudaError_t e = resident_ctas(kernel, threads, smem, &resident);
     if (e != cudaSuccess) return e;
     *grid = (unsigned)std::min<int64_t>(units, resident);
     return cudaSuccess;
 }
 
 template <typename K>
-static cudaError_t launch_persistent(K kernel, int64_t units, int threads, cudaStream_t s, const DeviceState& st,
+static cudaError_t launch_persistent(K kernel, int64_t units, int threads, size_t smem, cudaStream_t s, const DeviceState& st,
                                      const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
                                      const StepParams* d_steps, int nsteps) {
     unsigned grid = 0;
-    cudaError_t e = persistent_grid((const void*)kernel, threads, units, &grid);
+    cudaError_t e = persistent_grid((const void*)kernel, threads, smem, units, &grid);
     if (e != cudaSuccess) return e;
-    kernel<<<grid, threads, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);
+    kernel<<<grid, threads, smem, s>>>(st, pp, sp, sdf, d_steps, nsteps);
     return cudaGetLastError();
 }
 
@@ -741,8 +739,8 @@ static cudaError_t launch_fused_persistent(const DeviceState& st, const PhysPara
     if (units == 0) return cudaSuccess;
     const int threads = 32 * W;
 #define KAMI_PERSIST(KERNEL, CC)                                                                                 \
-    return jacobi ? launch_persistent(KERNEL<CC, true>, units, threads, s, st, pp, sp, sdf, d_steps, nsteps) \
-                  : launch_persistent(KERNEL<CC, false>, units, threads, s, st, pp, sp, sdf, d_steps, nsteps)
+    return jacobi ? launch_persistent(KERNEL<CC, true>, units, threads, park_bytes(CC, W), s, st, pp, sp, sdf, d_steps, nsteps) \
+                  : launch_persistent(KERNEL<CC, false>, units, threads, park_bytes(CC, W), s, st, pp, sp, sdf, d_steps, nsteps)
     if (group > 1) {
         if (group > 8 || st.num_tiles % group != 0) return cudaErrorInvalidValue;
         if (C == 2 && reg_cap == 120) KAMI_PERSIST(fused_persistent_group_kernel_r120, 2);
@@ -762,7 +760,7 @@ static cudaError_t launch_fused_persistent(const DeviceState& st, const PhysPara
 cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
                               int C, bool jacobi, int warps_per_block, cudaStream_t s, const StepParams* d_steps,
                               int nsteps, int reg_cap, int group, int launch_mode) {
-    if ((launch_mode & LAUNCH_PERSISTENT) && !(reg_cap == 2 && C == 4 && !jacobi && group <= 1))
+    if (launch_mode & LAUNCH_PERSISTENT)
         return launch_fused_persistent(st, pp, sp, sdf, C, jacobi, warps_per_block, s, d_steps, nsteps, reg_cap, group);
     if (group > 1) {
         if (group > 8 || st.num_tiles % group != 0) return cudaErrorInvalidValue;
@@ -772,9 +770,9 @@ cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const
 #define KAMI_GROUP_LAUNCH(KERNEL, CC)                                                                   \
     do {                                                                                                \
         if (jacobi)                                                                                     \
-            KERNEL<CC, true><<<gblocks, gthreads, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);             \
+            KERNEL<CC, true><<<gblocks, gthreads, park_bytes(CC, group), s>>>(st, pp, sp, sdf, d_steps, nsteps);             \
         else                                                                                            \
-            KERNEL<CC, false><<<gblocks, gthreads, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);            \
+            KERNEL<CC, false><<<gblocks, gthreads, park_bytes(CC, group), s>>>(st, pp, sp, sdf, d_steps, nsteps);            \
     } while (0)
         if (C == 2 && reg_cap == 120)
             KAMI_GROUP_LAUNCH(fused_group_kernel_r120, 2);
@@ -792,31 +790,30 @@ cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const
     int threads = 32 * warps_per_block;
     unsigned blocks = blocks_for(st.num_tiles, warps_per_block);
     if (blocks == 0) return cudaSuccess;
-    if (reg_cap == 2 && C == 4 && !jacobi) {
-        fused_step_kernel_x2<4><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, TapeView{}, d_steps, nsteps);
-        return cudaGetLastError();
-    }
     if (reg_cap == 168 && C == 4) {
         if (jacobi)
-            fused_step_kernel_r168<4, true><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, TapeView{}, d_steps, nsteps);
+            fused_step_kernel_r168<4, true><<<blocks, threads, park_bytes(4, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
+                nsteps);
         else
-            fused_step_kernel_r168<4, false><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, TapeView{}, d_steps, nsteps);
+            fused_step_kernel_r168<4, false><<<blocks, threads, park_bytes(4, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
+                nsteps);
         return cudaGetLastError();
     }
     if (reg_cap == 120 && C == 2) {
         if (jacobi)
-            fused_step_kernel_r120<2, true><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, TapeView{}, d_steps, nsteps);
+            fused_step_kernel_r120<2, true><<<blocks, threads, park_bytes(2, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
+                nsteps);
         else
-            fused_step_kernel_r120<2, false><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, TapeView{}, d_steps, nsteps);
+            fused_step_kernel_r120<2, false><<<blocks, threads, park_bytes(2, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
+                nsteps);
         return cudaGetLastError();
     }
-    const TapeView none{};
 #define KAMI_FUSED_CASE(CC)                                                                        \
     if (C == CC) {                                                                                 \
         if (jacobi)                                                                                \
-            fused_step_kernel<CC, true, false><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, none, d_steps, nsteps);  \
+            fused_step_kernel<CC, true><<<blocks, threads, park_bytes(CC, warps_per_block), s>>>(st, pp, sp, sdf, d_steps, nsteps);  \
         else                                                                                       \
-            fused_step_kernel<CC, false, false><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, none, d_steps, nsteps); \
+            fused_step_kernel<CC, false><<<blocks, threads, park_bytes(CC, warps_per_block), s>>>(st, pp, sp, sdf, d_steps, nsteps); \
         return cudaGetLastError();                                                                 \
     }
     KAMI_FUSED_CASE(2)

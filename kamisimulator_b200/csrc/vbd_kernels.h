@@ -28,9 +28,9 @@ cudaError_t launch_sweep_finish(const DeviceState& st, const float4* dx4, const 
 bool fused_supported(int C);
 // nsteps consecutive steps in one launch: parameters from d_steps[0..nsteps) (device), or sp when
 // d_steps is null (then nsteps must be 1).  group > 1: the layout's groups of `group` tiles, one CTA
-// of `group` warps each (warps_per_block and the packed variant do not apply).
+// of `group` warps each (warps_per_block does not apply).
 // launch_mode: 0 = one CTA per W tiles (or per group), scheduled by the hardware; LAUNCH_PERSISTENT =
-// resident CTAs loop over the tiles (fused_persistent_kernel; the packed variant has no persistent form).
+// resident CTAs loop over the tiles (fused_persistent_kernel).
 enum : int { LAUNCH_PERSISTENT = 1 };
 cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
                               int C, bool jacobi, int warps_per_block, cudaStream_t s, const StepParams* d_steps = nullptr,

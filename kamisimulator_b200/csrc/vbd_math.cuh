@@ -22,16 +22,19 @@ __device__ __forceinline__ void vbd_predict(float3 x, float3 v, float3 vlast, fl
         windx = pp.wind_peak * ((0.f < pw) ? pw : 0.f);
     }
     float3 ext = f3(pp.gx + windx, pp.gy, pp.gz) * pp.ext_mult;
-    dx = h * v;
+    // (written with fmaf: every kernel that predicts rounds alike)
+    dx = f3(__fmul_rn(h, v.x), __fmul_rn(h, v.y), __fmul_rn(h, v.z));
     y = v;
     if (inv_mass != 0.f) {
-        y = dx + (h * h) * ext;
-        float ext2 = dot3(ext, ext);
+        const float hh = __fmul_rn(h, h);
+        y = f3(fmaf(hh, ext.x, dx.x), fmaf(hh, ext.y, dx.y), fmaf(hh, ext.z, dx.z));
+        float ext2 = fmaf(ext.z, ext.z, fmaf(ext.x, ext.x, __fmul_rn(ext.y, ext.y)));
         if (ext2 > 0.f) {
             float3 acc = (v - vlast) * (1.f / last_h);
-            float s = dot3(acc, ext) / ext2;
+            float s = fmaf(acc.z, ext.z, fmaf(acc.x, ext.x, __fmul_rn(acc.y, ext.y))) / ext2;
             s = fminf(fmaxf(s, 0.f), 1.f);
-            dx = dx + (h * h * s) * ext;
+            const float c = __fmul_rn(hh, s);
+            dx = f3(fmaf(c, ext.x, dx.x), fmaf(c, ext.y, dx.y), fmaf(c, ext.z, dx.z));
         }
     }
 }
