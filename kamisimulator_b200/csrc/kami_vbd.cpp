@@ -9,8 +9,10 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <new>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -50,6 +52,66 @@ namespace kami {
 void set_last_error(const char* msg) { g_last_error = msg; }
 }  // namespace kami
 
+namespace {
+// Page-locked words that the device reports into: the status word, and a state buffer's clock.  One page
+// serves all handles of the process: page-locking it takes 0.3 to 0.5 ms (cudaHostAlloc 1 to 3 ms), half of
+// a small groom's whole kami_vbd_create.  It is made for the first handle and given back with the last.  A
+// read through it waits 11 us less than one through a pageable copy (1 us against 12 beyond the wait).
+struct Report {
+    int status;
+    float clock[4];
+    int pad[3];
+};
+struct ReportPool {
+    static constexpr int N = 4096 / (int)sizeof(Report);
+    std::mutex m;
+    Report* page = nullptr;
+    int used = 0;
+    bool taken[N] = {};
+    Report* take() {
+        std::lock_guard<std::mutex> g(m);
+        if (!page) {
+            void* p = std::aligned_alloc(4096, sizeof(Report) * N);
+            if (!p) return nullptr;
+            std::memset(p, 0, sizeof(Report) * N);
+            void* d = nullptr;
+            if (cudaHostRegister(p, sizeof(Report) * N, cudaHostRegisterMapped | cudaHostRegisterPortable) != cudaSuccess) {
+                cudaGetLastError();
+                std::free(p);
+                return nullptr;
+            }
+            if (cudaHostGetDevicePointer(&d, p, 0) != cudaSuccess || d != p) {  // kernels take the host's address
+                cudaGetLastError();
+                cudaHostUnregister(p);
+                std::free(p);
+                return nullptr;
+            }
+            page = (Report*)p;
+        }
+        for (int i = 0; i < N; i++)
+            if (!taken[i]) {
+                taken[i] = true;
+                used++;
+                return page + i;
+            }
+        return nullptr;
+    }
+    void give(Report* r) {  // nothing on a stream may still write to r
+        std::lock_guard<std::mutex> g(m);
+        taken[r - page] = false;
+        if (--used == 0) {
+            cudaHostUnregister(page);
+            std::free(page);
+            page = nullptr;
+        }
+    }
+};
+ReportPool& report_pool() {
+    static ReportPool* p = new ReportPool;  // outlives handles destroyed during process exit
+    return *p;
+}
+}  // namespace
+
 struct kami_vbd_solver {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -79,6 +141,7 @@ struct kami_vbd_solver {
     // entry of the run's first vertex; null when there is no Hair layout or it has 2^31 entries or more
     int4* d_hair_runs = nullptr;
     int* d_status = nullptr;
+    volatile Report* report = nullptr;  // null: the pool is full, these words are read through pageable copies
     float4* d_sdf = nullptr;
     SdfParams sdf{};
 
@@ -203,6 +266,7 @@ void release(kami_vbd_solver* h) {
                      h->d_strand_cta};
     for (void* p : cptrs)
         if (p) cudaFree(p);
+    if (h->report) report_pool().give((Report*)h->report);
     if (h->ev_a) cudaEventDestroy(h->ev_a);
     if (h->ev_b) cudaEventDestroy(h->ev_b);
     if (h->d_runs) cudaFree(h->d_runs);
@@ -232,10 +296,14 @@ kami_status on_stream(kami_vbd_solver* h, void* user_stream, F body) {
     return KAMI_OK;
 }
 
-kami_status check_status_word(kami_vbd_solver* h) {
+// Waits for the stream and reads the status word; `reported`: work on the stream already hands it out.
+kami_status check_status_word(kami_vbd_solver* h, bool reported = false) {
     int word = 0;
-    KAMI_CUDA(cudaMemcpyAsync(&word, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "status read");
+    int* dst = h->report ? (int*)&h->report->status : &word;
+    if (!reported)
+        KAMI_CUDA(cudaMemcpyAsync(dst, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "status read");
     KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+    if (h->report) word = h->report->status;
     if (word != 0) {
         KAMI_CUDA(cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream), "status reset");
         if (word & STATUS_NONFINITE)
@@ -261,6 +329,18 @@ kami_status stage_out(kami_vbd_solver* h, float* dst, int comps, int32_t memory)
     cudaMemcpyKind kind = memory == KAMI_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     KAMI_CUDA(cudaMemcpyAsync(dst, h->d_stage, bytes, kind, h->stream), "copy out");
     return KAMI_OK;
+}
+
+// Whether a kernel on the handle's device can read or write p itself: device memory of that device, or
+// managed memory.  Anything else goes through the staging buffer and the copy engine, as it always did.
+bool device_accessible(const kami_vbd_solver* h, const void* p) {
+    cudaPointerAttributes a{};
+    if (((uintptr_t)p & 3) != 0) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return (a.type == cudaMemoryTypeDevice && a.device == h->device) || a.type == cudaMemoryTypeManaged;
 }
 
 kami_status valid_handle(kami_vbd_solver* h) {
@@ -736,6 +816,7 @@ static kami_status create_impl(const kami_vbd_desc* descs, int32_t n, kami_vbd_h
     cudaError_t e = cudaStreamCreate(&h->stream);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_a, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_b, cudaEventDisableTiming);
+    if (e == cudaSuccess) h->report = report_pool().take();
     if (e == cudaSuccess) e = dalloc(&h->d_slot_of, h->nv);
     if (e == cudaSuccess) e = dalloc(&h->d_xm, S);
     if (e == cudaSuccess) e = dalloc(&h->d_vel, S);
@@ -857,6 +938,13 @@ kami_status kami_vbd_get_sizes(kami_vbd_handle h, int64_t* num_vertices, int32_t
 kami_status kami_vbd_set_positions_velocities(kami_vbd_handle h, const float* xyz, const float* vxyz, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (memory != KAMI_MEMORY_HOST && memory != KAMI_MEMORY_DEVICE) return fail(KAMI_ERR_INVALID_ARGUMENT, "bad memory kind");
+    if (memory == KAMI_MEMORY_DEVICE && (!xyz || device_accessible(h, xyz)) && (!vxyz || device_accessible(h, vxyz))) {
+        BoundaryArrays a;
+        if (xyz) a.add(h->d_xm, xyz, 3);
+        if (vxyz) a.add(h->d_vel, vxyz, 3);
+        if (a.n) KAMI_CUDA(launch_scatter_arrays(a, h->d_slot_of, h->nv, h->stream), "scatter positions and velocities");
+        return KAMI_OK;
+    }
     if (xyz) {
         KAMI_TRY(stage_in(h, xyz, 3, memory));
         KAMI_CUDA(launch_scatter3(h->d_stage, h->d_xm, h->d_slot_of, h->nv, h->stream), "scatter positions");
@@ -871,6 +959,16 @@ kami_status kami_vbd_set_positions_velocities(kami_vbd_handle h, const float* xy
 kami_status kami_vbd_get_positions_velocities(kami_vbd_handle h, float* xyz, float* vxyz, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (memory != KAMI_MEMORY_HOST && memory != KAMI_MEMORY_DEVICE) return fail(KAMI_ERR_INVALID_ARGUMENT, "bad memory kind");
+    if (memory == KAMI_MEMORY_DEVICE && (!xyz || device_accessible(h, xyz)) && (!vxyz || device_accessible(h, vxyz))) {
+        BoundaryArrays a;
+        if (xyz) a.add(h->d_xm, xyz, 3);
+        if (vxyz) a.add(h->d_vel, vxyz, 3);
+        if (a.n == 0) return check_status_word(h);
+        int* word = h->report ? (int*)&h->report->status : nullptr;
+        KAMI_CUDA(launch_gather_arrays(a, h->d_slot_of, h->nv, h->d_status, word, float4{}, nullptr, h->stream),
+                  "gather positions and velocities");
+        return check_status_word(h, word != nullptr);
+    }
     if (xyz) {
         KAMI_CUDA(launch_gather3(h->d_xm, h->d_stage, h->d_slot_of, h->nv, h->stream), "gather positions");
         KAMI_TRY(stage_out(h, xyz, 3, memory));
@@ -885,6 +983,13 @@ kami_status kami_vbd_get_positions_velocities(kami_vbd_handle h, float* xyz, flo
 static kami_status get4(kami_vbd_solver* h, const float4* src, float* dst, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (!dst) return fail(KAMI_ERR_INVALID_ARGUMENT, "null output");
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, dst)) {
+        BoundaryArrays a;
+        a.add(const_cast<float4*>(src), dst, 4);
+        KAMI_CUDA(launch_gather_arrays(a, h->d_slot_of, h->nv, nullptr, nullptr, float4{}, nullptr, h->stream), "gather");
+        KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+        return KAMI_OK;
+    }
     KAMI_CUDA(launch_gather4(src, (float4*)h->d_stage, h->d_slot_of, h->nv, h->stream), "gather");
     KAMI_TRY(stage_out(h, dst, 4, memory));
     KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
@@ -893,6 +998,12 @@ static kami_status get4(kami_vbd_solver* h, const float4* src, float* dst, int32
 static kami_status set4(kami_vbd_solver* h, float4* dst, const float* src, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (!src) return fail(KAMI_ERR_INVALID_ARGUMENT, "null input");
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, src)) {
+        BoundaryArrays a;
+        a.add(dst, src, 4);
+        KAMI_CUDA(launch_scatter_arrays(a, h->d_slot_of, h->nv, h->stream), "scatter");
+        return KAMI_OK;
+    }
     KAMI_TRY(stage_in(h, src, 4, memory));
     KAMI_CUDA(launch_scatter4((const float4*)h->d_stage, dst, h->d_slot_of, h->nv, h->stream), "scatter");
     return KAMI_OK;
@@ -1533,9 +1644,7 @@ kami_status kami_vbd_get_tiles_per_group(kami_vbd_handle h, int32_t* tiles_per_g
 // The tape window's slots [s0, s0 + n) and the slot -> vertex map for the scatters and gathers of
 // kami_vbd_backward and kami_vbd_restore_tape_window; *vert_of stays null when the window covers the
 // whole groom.
-static kami_status window_slots(kami_vbd_solver* h, const int64_t** vert_of, int64_t* s0, int64_t* n) {
-    *vert_of = nullptr;
-    if (h->win_begin == 0 && h->win_end >= h->layout.num_tiles) return KAMI_OK;
+static kami_status slot_vertices(kami_vbd_solver* h) {  // builds d_vert_of for the current layout
     if (!h->d_vert_of || h->vert_of_C != h->layout.C || h->vert_of_K != h->layout.K) {
         if (h->d_vert_of) cudaFree(h->d_vert_of);
         h->d_vert_of = nullptr;
@@ -1544,6 +1653,12 @@ static kami_status window_slots(kami_vbd_solver* h, const int64_t** vert_of, int
         h->vert_of_C = h->layout.C;
         h->vert_of_K = h->layout.K;
     }
+    return KAMI_OK;
+}
+static kami_status window_slots(kami_vbd_solver* h, const int64_t** vert_of, int64_t* s0, int64_t* n) {
+    *vert_of = nullptr;
+    if (h->win_begin == 0 && h->win_end >= h->layout.num_tiles) return KAMI_OK;
+    KAMI_TRY(slot_vertices(h));
     const int64_t T = 32LL * h->layout.C;
     *vert_of = h->d_vert_of;
     *s0 = h->win_begin * T;
@@ -1620,12 +1735,20 @@ kami_status kami_vbd_backward(kami_vbd_handle h, float* adj_x, float* adj_v, flo
     const int64_t* wv = nullptr;
     int64_t ws0 = 0, wn = 0;
     if (memory == KAMI_MEMORY_DEVICE) KAMI_TRY(window_slots(h, &wv, &ws0, &wn));
+    const bool direct = memory == KAMI_MEMORY_DEVICE && device_accessible(h, adj_x) && device_accessible(h, adj_v) &&
+                        device_accessible(h, adj_vlast) && device_accessible(h, adj_q);
     if (wv) {
         for (int a = 0; a < 3; a++) {
             KAMI_CUDA(cudaMemsetAsync(adj3[a] + ws0, 0, sizeof(float4) * wn, h->stream), "adjoint reset");
             KAMI_CUDA(launch_scatter_slots(ins3[a], adj3[a], wv, ws0, wn, 3, h->stream), "scatter adjoint");
         }
         KAMI_CUDA(launch_scatter_slots(adj_q, h->d_gq, wv, ws0, wn, 4, h->stream), "scatter adjoint");
+    } else if (direct) {
+        BoundaryArrays a;
+        for (int k = 0; k < 3; k++) a.add(adj3[k], ins3[k], 3);
+        a.add(h->d_gq, adj_q, 4);
+        KAMI_TRY(slot_vertices(h));
+        KAMI_CUDA(launch_fill_arrays(a, h->d_vert_of, (int64_t)S, h->stream), "scatter adjoint");
     } else {
         for (int a = 0; a < 3; a++) {
             KAMI_CUDA(cudaMemsetAsync(adj3[a], 0, sizeof(float4) * S, h->stream), "adjoint reset");
@@ -1653,6 +1776,12 @@ kami_status kami_vbd_backward(kami_vbd_handle h, float* adj_x, float* adj_v, flo
         for (int a = 0; a < 3; a++)
             KAMI_CUDA(launch_gather_slots(adj3[a], ins3[a], wv, ws0, wn, 3, h->stream), "gather adjoint");
         KAMI_CUDA(launch_gather_slots(h->d_gq, adj_q, wv, ws0, wn, 4, h->stream), "gather adjoint");
+    } else if (direct) {
+        BoundaryArrays a;
+        for (int k = 0; k < 3; k++) a.add(adj3[k], ins3[k], 3);
+        a.add(h->d_gq, adj_q, 4);
+        KAMI_CUDA(launch_gather_arrays(a, h->d_slot_of, h->nv, nullptr, nullptr, float4{}, nullptr, h->stream),
+                  "gather adjoint");
     } else {
         for (int a = 0; a < 3; a++) {
             KAMI_CUDA(launch_gather3(adj3[a], h->d_stage, h->d_slot_of, h->nv, h->stream), "gather adjoint");
@@ -1871,6 +2000,23 @@ kami_status kami_vbd_get_state(kami_vbd_handle h, void* dst, size_t bytes, int32
     if (!dst || bytes < need) return fail(KAMI_ERR_INVALID_ARGUMENT, "state buffer must hold %zu bytes", need);
     float* f = (float*)dst;
     const int64_t nv = h->nv;
+    // the fourth word holds the substep counter (uint32 bits), which paces hair-hair detection
+    const uint32_t ctr = (uint32_t)h->counter;
+    float ctr_f;
+    std::memcpy(&ctr_f, &ctr, 4);
+    const float clk[4] = {h->h, h->last_h, h->time, ctr_f};
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, dst) && nv > 0) {
+        BoundaryArrays a;
+        a.add(h->d_xm, f, 3);
+        a.add(h->d_vel, f + 3 * nv, 3);
+        a.add(h->d_vlast, f + 6 * nv, 3);
+        a.add(h->d_q, f + 9 * nv, 4);
+        KAMI_CUDA(launch_gather_arrays(a, h->d_slot_of, nv, nullptr, nullptr, make_float4(clk[0], clk[1], clk[2], clk[3]),
+                                       f + 13 * nv, h->stream),
+                  "gather state");
+        KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+        return KAMI_OK;
+    }
     cudaMemcpyKind kind = memory == KAMI_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     const float4* srcs[3] = {h->d_xm, h->d_vel, h->d_vlast};
     for (int a = 0; a < 3; a++) {
@@ -1880,11 +2026,6 @@ kami_status kami_vbd_get_state(kami_vbd_handle h, void* dst, size_t bytes, int32
     KAMI_CUDA(launch_gather4(h->d_q, (float4*)h->d_stage, h->d_slot_of, nv, h->stream), "gather state");
     KAMI_CUDA(cudaMemcpyAsync(f + 9 * nv, h->d_stage, sizeof(float) * 4 * nv, kind, h->stream), "state copy");
     KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
-    // the fourth word holds the substep counter (uint32 bits), which paces hair-hair detection
-    const uint32_t ctr = (uint32_t)h->counter;
-    float ctr_f;
-    std::memcpy(&ctr_f, &ctr, 4);
-    const float clk[4] = {h->h, h->last_h, h->time, ctr_f};
     if (memory == KAMI_MEMORY_DEVICE)
         KAMI_CUDA(cudaMemcpy(f + 13 * nv, clk, sizeof(clk), cudaMemcpyHostToDevice), "state clock");
     else
@@ -1901,18 +2042,30 @@ kami_status kami_vbd_set_state(kami_vbd_handle h, const void* src, size_t bytes,
     const int64_t nv = h->nv;
     cudaMemcpyKind kind = memory == KAMI_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     float4* dsts[3] = {h->d_xm, h->d_vel, h->d_vlast};
-    for (int a = 0; a < 3; a++) {
-        KAMI_CUDA(cudaMemcpyAsync(h->d_stage, f + 3 * nv * a, sizeof(float) * 3 * nv, kind, h->stream), "state copy");
-        KAMI_CUDA(launch_scatter3(h->d_stage, dsts[a], h->d_slot_of, nv, h->stream), "scatter state");
-    }
-    KAMI_CUDA(cudaMemcpyAsync(h->d_stage, f + 9 * nv, sizeof(float) * 4 * nv, kind, h->stream), "state copy");
-    KAMI_CUDA(launch_scatter4((const float4*)h->d_stage, h->d_q, h->d_slot_of, nv, h->stream), "scatter state");
-    KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
     float clk[4];
-    if (memory == KAMI_MEMORY_DEVICE)
-        KAMI_CUDA(cudaMemcpy(clk, f + 13 * nv, sizeof(clk), cudaMemcpyDeviceToHost), "state clock");
-    else
-        std::memcpy(clk, f + 13 * nv, sizeof(clk));
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, src)) {
+        BoundaryArrays a;
+        for (int k = 0; k < 3; k++) a.add(dsts[k], f + 3 * nv * k, 3);
+        a.add(h->d_q, f + 9 * nv, 4);
+        KAMI_CUDA(launch_scatter_arrays(a, h->d_slot_of, nv, h->stream), "scatter state");
+        float* dst = h->report ? (float*)h->report->clock : clk;
+        KAMI_CUDA(cudaMemcpyAsync(dst, f + 13 * nv, sizeof(clk), cudaMemcpyDeviceToHost, h->stream), "state clock");
+        KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+        if (h->report)
+            for (int k = 0; k < 4; k++) clk[k] = h->report->clock[k];
+    } else {
+        for (int a = 0; a < 3; a++) {
+            KAMI_CUDA(cudaMemcpyAsync(h->d_stage, f + 3 * nv * a, sizeof(float) * 3 * nv, kind, h->stream), "state copy");
+            KAMI_CUDA(launch_scatter3(h->d_stage, dsts[a], h->d_slot_of, nv, h->stream), "scatter state");
+        }
+        KAMI_CUDA(cudaMemcpyAsync(h->d_stage, f + 9 * nv, sizeof(float) * 4 * nv, kind, h->stream), "state copy");
+        KAMI_CUDA(launch_scatter4((const float4*)h->d_stage, h->d_q, h->d_slot_of, nv, h->stream), "scatter state");
+        KAMI_CUDA(cudaStreamSynchronize(h->stream), "cudaStreamSynchronize");
+        if (memory == KAMI_MEMORY_DEVICE)
+            KAMI_CUDA(cudaMemcpy(clk, f + 13 * nv, sizeof(clk), cudaMemcpyDeviceToHost), "state clock");
+        else
+            std::memcpy(clk, f + 13 * nv, sizeof(clk));
+    }
     h->h = clk[0];
     h->last_h = clk[1];
     h->time = clk[2];

@@ -468,6 +468,61 @@ __global__ void gather4_kernel(const float4* __restrict__ src, float4* __restric
     if (i >= nv) return;
     dst[i] = src[slot_of[i]];
 }
+// Several of a call's arrays at once, between the caller's device arrays and the tile slots: one launch,
+// and each vertex's slot is looked up once.  Memory bound: 8 B of index and 28 B an array and vertex
+// (a step of 640,000 vertices and the read of its positions and velocities: 129 us of wall time with two
+// gathers into a staging buffer and two copies out of it, 104 with this, of which 11 are the status word's
+// pageable copy; 64 x 32 vertices 40 and 20).  Boundary arrays are read and written as floats (any 4-byte alignment).  The
+// gather's first thread also hands out what the call reports beside them: the status word and a clock.
+__global__ void gather_arrays_kernel(BoundaryArrays a, const int64_t* __restrict__ slot_of, int64_t nv,
+                                     const int* status, int* status_out, float4 clock, float* clock_out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        if (status_out) *status_out = *status;
+        if (clock_out) {
+            clock_out[0] = clock.x;
+            clock_out[1] = clock.y;
+            clock_out[2] = clock.z;
+            clock_out[3] = clock.w;
+        }
+    }
+    if (i >= nv) return;
+    const int64_t g = slot_of[i];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (k >= a.n) break;
+        const float4 t = a.slots[k][g];
+        float* o = a.flat[k] + a.comps[k] * i;
+        o[0] = t.x;
+        o[1] = t.y;
+        o[2] = t.z;
+        if (a.comps[k] == 4) o[3] = t.w;
+    }
+}
+__global__ void scatter_arrays_kernel(BoundaryArrays a, const int64_t* __restrict__ slot_of, int64_t nv) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nv) return;
+    const int64_t g = slot_of[i];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (k >= a.n) break;
+        const float* f = a.flat[k] + a.comps[k] * i;
+        a.slots[k][g] = make_float4(f[0], f[1], f[2], a.comps[k] == 4 ? f[3] : a.slots[k][g].w);
+    }
+}
+// The same into every slot, zero in padding slots (the adjoint's buffers); vert_of as below.
+__global__ void fill_arrays_kernel(BoundaryArrays a, const int64_t* __restrict__ vert_of, int64_t num_slots) {
+    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= num_slots) return;
+    const int64_t i = vert_of[g];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        if (k >= a.n) break;
+        const float* f = a.flat[k] + a.comps[k] * i;
+        a.slots[k][g] = i < 0 ? make_float4(0.f, 0.f, 0.f, 0.f)
+                              : make_float4(f[0], f[1], f[2], a.comps[k] == 4 ? f[3] : 0.f);
+    }
+}
 // Tape windows: the slots [s0, s0 + n) of a window and the boundary vertices they hold (vert_of: the
 // vertex of each slot, -1 for padding).  Slot side in tile order, boundary side read and written as
 // floats (its 4-vectors need not start on 16-byte boundaries, e.g. the orientations inside a state
@@ -875,6 +930,22 @@ cudaError_t launch_scatter4(const float4* src, float4* dst, const int64_t* slot_
 cudaError_t launch_gather4(const float4* src, float4* dst, const int64_t* slot_of, int64_t nv, cudaStream_t s) {
     if (nv == 0) return cudaSuccess;
     gather4_kernel<<<blocks_for(nv, 256), 256, 0, s>>>(src, dst, slot_of, nv);
+    return cudaGetLastError();
+}
+cudaError_t launch_gather_arrays(const BoundaryArrays& a, const int64_t* slot_of, int64_t nv, const int* status,
+                                 int* status_out, float4 clock, float* clock_out, cudaStream_t s) {
+    if (nv == 0) return cudaSuccess;
+    gather_arrays_kernel<<<blocks_for(nv, 256), 256, 0, s>>>(a, slot_of, nv, status, status_out, clock, clock_out);
+    return cudaGetLastError();
+}
+cudaError_t launch_scatter_arrays(const BoundaryArrays& a, const int64_t* slot_of, int64_t nv, cudaStream_t s) {
+    if (nv == 0) return cudaSuccess;
+    scatter_arrays_kernel<<<blocks_for(nv, 256), 256, 0, s>>>(a, slot_of, nv);
+    return cudaGetLastError();
+}
+cudaError_t launch_fill_arrays(const BoundaryArrays& a, const int64_t* vert_of, int64_t num_slots, cudaStream_t s) {
+    if (num_slots == 0) return cudaSuccess;
+    fill_arrays_kernel<<<blocks_for(num_slots, 256), 256, 0, s>>>(a, vert_of, num_slots);
     return cudaGetLastError();
 }
 cudaError_t launch_vert_of(const int64_t* slot_of, int64_t* vert_of, int64_t nv, int64_t num_slots, cudaStream_t s) {
