@@ -63,3 +63,35 @@ def test_baked_head_drives_the_solver_like_the_analytic_sphere():
     assert np.abs(xs[0] - xs[1]).max() <= 3e-4
     moved = np.abs(xs[1] - g.positions).max()
     assert moved > 1e-3  # the SDF pass pushed vertices out by millimetres
+
+
+def _mesh_of(kind):
+    rng = np.random.default_rng(11)
+    if kind == "tetrahedron":  # fewer triangles than a cluster holds
+        return np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1]], np.float32) * np.float32(0.1), \
+            np.array([[0, 2, 1], [0, 1, 3], [1, 2, 3], [0, 3, 2]], np.int32)
+    V, T = synth.icosphere(3, 0.09)
+    if kind == "slivers":  # clusters that may not be skipped beside clusters that may
+        V = (V * np.array([1.0, 1.0, 1e-3])).astype(np.float32)
+    elif kind == "away":
+        V = (V + np.float32([3.0, -2.0, 1.0])).astype(np.float32)
+    elif kind == "rough":
+        V = (V + rng.normal(0, 2e-3, V.shape)).astype(np.float32)
+    return V, T
+
+
+@pytest.mark.parametrize("kind,dims,pad", [
+    ("tetrahedron", (1, 1, 1), 0.05), ("tetrahedron", (5, 3, 7), 0.05), ("sphere", (9, 6, 3), 0.02),
+    ("sphere", (8, 8, 4), 3.0), ("slivers", (13, 11, 10), 0.05), ("away", (10, 9, 5), 0.05), ("rough", (12, 7, 9), 0.1)])
+def test_gpu_bake_skips_no_nearest_triangle(kind, dims, pad):
+    """Clusters of triangles are skipped by a bound on their distance: the magnitudes still are the FP64
+    distances over all triangles.  Tolerance: the node and the closest point are FP32 coordinates (a few units
+    in the last place of the largest one, 6e-8 of it), and the weights of an interior closest point are off by
+    up to 72 u (L D / 2A)^2 of the longest edge L, at a right angle to the distance; taken as 2e-6 + 1e-6 of
+    the largest coordinate, and for a point displaced by s at distance d, s^2 / 2d is far below that here."""
+    V, T = _mesh_of(kind)
+    lo, hi = V.min(0) - np.float32(pad), V.max(0) + np.float32(pad)
+    g = vbd.bake_sdf(V, T, dims, lo, hi)
+    phi, _ = orc.sdf_bake(V, T, dims, g.grid_min, g.grid_max)
+    big = max(np.abs(lo).max(), np.abs(hi).max())
+    assert np.abs(np.abs(g.phi) - np.abs(phi)).max() <= 2e-6 + 1e-6 * big
