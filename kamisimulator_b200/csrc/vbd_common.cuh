@@ -213,6 +213,20 @@ __host__ __device__ __forceinline__ float3 qrotate(float4 r, float3 v) {
     return r.w * a + cross3(qv, a) + c * qv;
 }
 
+// Chained launches (programmatic dependent launch): a kernel launched with launch_chained may start before
+// the kernel ahead of it in the stream has ended.  grid_wait() returns when that one is complete and its
+// writes are visible; before it, only what no kernel still running can write may be read.  Every kernel of
+// such a chain calls both, grid_wait first, so at most two of its kernels are in flight and what was complete
+// before the kernel ahead passed its own grid_wait is safe to read at once.  Both do nothing in a kernel
+// launched the ordinary way.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// A read that stays behind grid_wait (volatile) and sees other SMs' writes (L2).
+__device__ __forceinline__ float4 load_fresh(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ float3 shfl_up3(float3 v, int d) {
     return f3(__shfl_up_sync(0xffffffffu, v.x, d), __shfl_up_sync(0xffffffffu, v.y, d), __shfl_up_sync(0xffffffffu, v.z, d));
 }

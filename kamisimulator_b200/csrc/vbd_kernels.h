@@ -7,6 +7,24 @@
 
 namespace kami {
 
+// A launch that may overlap the kernel ahead of it (see grid_wait in vbd_common.cuh); the kernel ahead must be
+// one that calls grid_wait and grid_release.
+template <class... P, class... A>
+cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                           A... args) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    c.numAttrs = chained ? 1 : 0;
+    return cudaLaunchKernelEx(&c, kernel, static_cast<P>(args)...);
+}
+
 cudaError_t launch_sweep_predict(const DeviceState& st, float4* y4, float4* dx4, const StepParams* d_sp,
                                  const PhysParams& pp, int64_t num_slots, cudaStream_t s);
 // conn_dx: the partners' dx for tied vertices (st.conn), the iteration's starting values
@@ -16,10 +34,11 @@ cudaError_t launch_sweep_position(const DeviceState& st, const float4* y4, const
 // One iteration (colour2: both position sweeps, both orientation sweeps; jacobi: the position and
 // the orientation sweep) in one launch, one block per tile of up to 1024 slots: reads dx_in, writes
 // dx_out; q in place for colour2 (q_in == q_out), into q_out for jacobi (sweep_iteration_supported).
+// chained: only behind another iteration of the same substep (it reads y4 ahead of grid_wait).
 bool sweep_iteration_supported(int C);
 cudaError_t launch_sweep_iteration(const DeviceState& st, const float4* y4, const float4* q_in, float4* q_out,
                                    const float4* dx_in, float4* dx_out, const StepParams* d_sp, const PhysParams& pp,
-                                   int C, bool jacobi, cudaStream_t s);
+                                   int C, bool jacobi, bool chained, cudaStream_t s);
 cudaError_t launch_sweep_orientation(const DeviceState& st, const float4* dx4, const float4* q_in, float4* q_out, int C,
                                      int colour, bool jacobi, cudaStream_t s);
 cudaError_t launch_sweep_finish(const DeviceState& st, const float4* dx4, const StepParams* d_sp, const PhysParams& pp,
@@ -59,7 +78,7 @@ cudaError_t launch_coll_steplimit(const DeviceState& st, const float4* dx4, cons
 // q in place.  Tiles of up to 1024 slots (coll_iteration_supported).
 bool coll_iteration_supported(int C);
 cudaError_t launch_coll_iteration(const DeviceState& st, const float4* y4, float4* q, const float4* snap, float4* dx_out,
-                                  const StepParams* d_sp, const PhysParams& pp, const CollParams& cp, cudaStream_t s);
+                                  const StepParams* d_sp, const PhysParams& pp, const CollParams& cp, bool chained, cudaStream_t s);
 cudaError_t launch_sweep_position_coll(const DeviceState& st, const float4* y4, const float4* q, const float4* dx_in,
                                        float4* dx_out, const float4* snap, const StepParams* d_sp, const PhysParams& pp,
                                        const CollParams& cp, int colour, bool jacobi, cudaStream_t s);
