@@ -381,19 +381,21 @@ kami_status build_sweep_graph(kami_vbd_solver* h, int substeps) {
     cudaError_t err = cudaSuccess;
     const size_t b4 = sizeof(float4) * h->layout.num_slots;
     for (int sub = 0; sub < substeps && err == cudaSuccess; sub++) {
-        err = launch_sweep_predict(st, h->d_y, h->d_dx, h->d_step, h->pp, h->layout.num_slots, s);
+        err = launch_sweep_predict(st, h->d_y, h->d_dx, h->d_step, h->pp, h->layout.num_slots, sub > 0, s);
         if (h->hair_hair) {
             if (err == cudaSuccess && detect[sub]) err = launch_coll_detect(st, h->d_dx, h->cp, s);
-            if (err == cudaSuccess) err = launch_coll_steplimit(st, h->d_dx, h->cp, s);
+            if (err == cudaSuccess) err = launch_coll_steplimit(st, h->d_dx, h->cp, true, s);
         }
         float4* dx_cur = h->d_dx;
         float4* dx_alt = h->d_dx2;
         float4* q_cur = h->d_q;
         float4* q_alt = h->d_q2;
+        bool chained = false;  // whether the latest launch lets the next one overlap it (grid_wait)
         for (int it = 0; it < h->pp.num_itr && err == cudaSuccess; it++) {
             if (jac && !h->hair_hair && h->layout.K == 1 && sweep_iteration_supported(C)) {
                 // the whole iteration in one launch: dx_cur -> dx_alt, q_cur -> q_alt
-                err = launch_sweep_iteration(st, h->d_y, q_cur, q_alt, dx_cur, dx_alt, h->d_step, h->pp, C, true, it > 0, s);
+                err = launch_sweep_iteration(st, h->d_y, q_cur, q_alt, dx_cur, dx_alt, h->d_step, h->pp, C, true, true, s);
+                chained = true;
                 std::swap(dx_cur, dx_alt);
                 std::swap(q_cur, q_alt);
             } else if (jac) {
@@ -411,6 +413,7 @@ kami_status build_sweep_graph(kami_vbd_solver* h, int substeps) {
                 // d_dx and d_snap (a colour2 handle has no d_dx2; its snapshot buffer is free here)
                 float4* other = dx_cur == h->d_dx ? h->d_snap : h->d_dx;
                 err = launch_coll_iteration(st, h->d_y, q_cur, dx_cur, other, h->d_step, h->pp, h->cp, it > 0, s);
+                chained = true;
                 dx_cur = other;
             } else if (h->hair_hair) {
                 err = cudaMemcpyAsync(h->d_snap, dx_cur, b4, cudaMemcpyDeviceToDevice, s);  // partners' dx
@@ -422,7 +425,8 @@ kami_status build_sweep_graph(kami_vbd_solver* h, int substeps) {
             } else if (h->layout.K == 1 && sweep_iteration_supported(C) && h->d_snap) {
                 // the whole iteration in one launch, from dx_cur into the other of d_dx and d_snap
                 float4* other = dx_cur == h->d_dx ? h->d_snap : h->d_dx;
-                err = launch_sweep_iteration(st, h->d_y, q_cur, q_cur, dx_cur, other, h->d_step, h->pp, C, false, it > 0, s);
+                err = launch_sweep_iteration(st, h->d_y, q_cur, q_cur, dx_cur, other, h->d_step, h->pp, C, false, true, s);
+                chained = true;
                 dx_cur = other;
             } else {
                 if (h->d_conn)  // the tied partners' dx at the start of the iteration
@@ -434,10 +438,13 @@ kami_status build_sweep_graph(kami_vbd_solver* h, int substeps) {
                     err = launch_sweep_orientation(st, dx_cur, q_cur, q_cur, C, c, false, s);
             }
         }
-        if (err == cudaSuccess && q_cur != h->d_q)
+        if (err == cudaSuccess && q_cur != h->d_q) {
             err = cudaMemcpyAsync(h->d_q, q_cur, sizeof(float4) * h->layout.num_slots, cudaMemcpyDeviceToDevice, s);
+            chained = false;
+        }
         if (err == cudaSuccess)
-            err = launch_sweep_finish(st, dx_cur, h->d_step, h->pp, h->sdf, sub == substeps - 1, h->layout.num_slots, s);
+            err = launch_sweep_finish(st, dx_cur, h->d_step, h->pp, h->sdf, sub == substeps - 1, h->layout.num_slots,
+                                      chained, s);
     }
     cudaGraph_t g = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(s, &g);

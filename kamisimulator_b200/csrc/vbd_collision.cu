@@ -73,8 +73,12 @@ __device__ __forceinline__ float3 solve_sym3(const float H[6], float3 f) {
 
 // ---- detection --------------------------------------------------------------------------------
 
-__global__ void coll_box_kernel(DeviceState st, const float4* __restrict__ dx4, CollParams cp) {
+// (The detection's launches are chained: each kernel is short, and each needs all of the one before it.)
+__global__ void coll_box_kernel(DeviceState st, const float4* dx4, CollParams cp) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
+    grid_release();
+    for (int64_t k = g; k < 1LL << cp.table_bits; k += (int64_t)gridDim.x * blockDim.x) cp.count[k] = 0;
     float ext = 0.f;
     if (g < cp.num_slots) {
         const uint32_t fl = __float_as_uint(st.prm[g].w);
@@ -113,6 +117,8 @@ __device__ __forceinline__ bool box_cell(const CollParams& cp, int64_t g, int3& 
 
 __global__ void coll_hash_kernel(CollParams cp) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
+    grid_release();
     if (g >= cp.num_slots) return;
     int3 ci;
     if (!box_cell(cp, g, ci)) {
@@ -127,6 +133,8 @@ __global__ void coll_hash_kernel(CollParams cp) {
 
 __global__ void coll_scatter_kernel(CollParams cp) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
+    grid_release();
     if (g >= cp.num_slots) return;
     const uint32_t h = cp.cell[g];
     if (h == NO_CELL) return;
@@ -152,6 +160,8 @@ __global__ void __launch_bounds__(32 * kQueryWarps, 9) coll_query_kernel(DeviceS
     __shared__ int32_t s_lst[kQueryWarps][MAX_CONTACTS], s_key[kQueryWarps][MAX_CONTACTS];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t g = (int64_t)blockIdx.x * kQueryWarps + w;
+    grid_wait();
+    grid_release();
     if (g >= cp.num_slots) return;  // uniform per warp
     // the segment's own operands are loaded before the bucket look-ups, so that they are in flight
     // beside them instead of after them
@@ -272,6 +282,8 @@ __global__ void __launch_bounds__(32 * kQueryWarps, 9) coll_query_kernel(DeviceS
 // Exclusive scan of int32 counts, 4096 per block (1024 threads x 4): per-block scan + block sums.
 __global__ void __launch_bounds__(1024) scan_block_kernel(const int32_t* in, int32_t* out, int32_t* sums, int64_t n) {
     __shared__ int32_t warp_tot[32];
+    grid_wait();
+    grid_release();
     const int64_t base = (int64_t)blockIdx.x * 4096 + (int64_t)threadIdx.x * 4;
     int32_t v[4];
     for (int i = 0; i < 4; i++) v[i] = (base + i < n) ? in[base + i] : 0;
@@ -302,26 +314,33 @@ __global__ void __launch_bounds__(1024) scan_block_kernel(const int32_t* in, int
     }
 }
 
-__global__ void scan_add_kernel(int32_t* out, const int32_t* offs, int64_t n) {
+__global__ void scan_add_kernel(int32_t* out, const int32_t* offs, int64_t n, int32_t* copy) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] += offs[i / 4096];
+    grid_wait();
+    grid_release();
+    if (i >= n) return;
+    const int32_t v = out[i] + offs[i / 4096];
+    out[i] = v;
+    if (copy) copy[i] = v;
 }
 
-cudaError_t exclusive_scan(const int32_t* in, int32_t* out, int64_t n, int32_t* tmp, cudaStream_t s) {
+// copy (may be null): the result once more
+cudaError_t exclusive_scan(const int32_t* in, int32_t* out, int64_t n, int32_t* tmp, int32_t* copy, cudaStream_t s) {
     const int64_t blocks = (n + 4095) / 4096;
-    scan_block_kernel<<<(unsigned)blocks, 1024, 0, s>>>(in, out, tmp, n);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || blocks == 1) return e;
-    e = exclusive_scan(tmp, tmp, blocks, tmp + blocks, s);
+    cudaError_t e = launch_chained(true, scan_block_kernel, (unsigned)blocks, 1024, 0, s, in, out, tmp, n);
     if (e != cudaSuccess) return e;
-    scan_add_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, tmp, n);
-    return cudaGetLastError();
+    if (blocks > 1 && (e = exclusive_scan(tmp, tmp, blocks, tmp + blocks, nullptr, s)) != cudaSuccess) return e;
+    if (blocks == 1 && !copy) return cudaSuccess;
+    if (blocks == 1) return cudaMemcpyAsync(copy, out, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, s);
+    return launch_chained(true, scan_add_kernel, (unsigned)((n + 255) / 256), 256, 0, s, out, tmp, n, copy);
 }
 
 // ---- step limit ---------------------------------------------------------------------------------
 
-__global__ void coll_steplimit_kernel(DeviceState st, const float4* __restrict__ dx4, CollParams cp) {
+__global__ void coll_steplimit_kernel(DeviceState st, const float4* dx4, CollParams cp) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
+    grid_release();
     if (g >= cp.num_slots) return;
     const uint32_t fl = __float_as_uint(st.prm[g].w);
     float min_dist = INFINITY;
@@ -949,21 +968,16 @@ cudaError_t launch_coll_detect(const DeviceState& st, const float4* dx4, const C
     if (e != cudaSuccess) return e;
     coll_box_kernel<<<blocks_of(S, 256), 256, 0, s>>>(st, dx4, cp);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(cp.count, 0, sizeof(int32_t) * table, s)) != cudaSuccess) return e;
-    coll_hash_kernel<<<blocks_of(S, 256), 256, 0, s>>>(cp);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = exclusive_scan(cp.count, cp.start, table, cp.scan_tmp, s)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(cp.cursor, cp.start, sizeof(int32_t) * table, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-        return e;
-    coll_scatter_kernel<<<blocks_of(S, 256), 256, 0, s>>>(cp);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    coll_query_kernel<<<blocks_of(S, kQueryWarps), 32 * kQueryWarps, 0, s>>>(st, cp);
-    return cudaGetLastError();
+    if ((e = launch_chained(true, coll_hash_kernel, blocks_of(S, 256), 256, 0, s, cp)) != cudaSuccess) return e;
+    if ((e = exclusive_scan(cp.count, cp.start, table, cp.scan_tmp, cp.cursor, s)) != cudaSuccess) return e;
+    // (a table of one scan block ends in a copy, not in a kernel)
+    if ((e = launch_chained(table > 4096, coll_scatter_kernel, blocks_of(S, 256), 256, 0, s, cp)) != cudaSuccess) return e;
+    return launch_chained(true, coll_query_kernel, blocks_of(S, kQueryWarps), 32 * kQueryWarps, 0, s, st, cp);
 }
 
-cudaError_t launch_coll_steplimit(const DeviceState& st, const float4* dx4, const CollParams& cp, cudaStream_t s) {
-    coll_steplimit_kernel<<<blocks_of(cp.num_slots, 256), 256, 0, s>>>(st, dx4, cp);
-    return cudaGetLastError();
+cudaError_t launch_coll_steplimit(const DeviceState& st, const float4* dx4, const CollParams& cp, bool chained,
+                                  cudaStream_t s) {
+    return launch_chained(chained, coll_steplimit_kernel, blocks_of(cp.num_slots, 256), 256, 0, s, st, dx4, cp);
 }
 
 bool coll_iteration_supported(int C) { return C % 2 == 0 && C >= 2 && 32 * C <= 1024; }

@@ -28,9 +28,11 @@ namespace kami {
 // ==========================================================================================
 
 // initItr for every slot; writes y4 = (y, 1/(invMass h^2)), dx4 = (dx, 0), vlast = v.
-__global__ void sweep_predict_kernel(DeviceState st, float4* __restrict__ y4, float4* __restrict__ dx4,
-                                     const StepParams* __restrict__ spp, PhysParams pp, int64_t num_slots) {
+__global__ void sweep_predict_kernel(DeviceState st, float4* y4, float4* dx4, const StepParams* __restrict__ spp,
+                                     PhysParams pp, int64_t num_slots) {
     int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
+    grid_release();
     if (g >= num_slots) return;
     const StepParams sp = *spp;
     float4 xm = st.xm[g];
@@ -162,9 +164,8 @@ __global__ void sweep_orientation_kernel(DeviceState st, const float4* __restric
 // the state is read once per iteration instead of once per sweep.  dx goes to dx_out, q is updated
 // in place.
 // Bound by latency: a launch, the loads, four dependent sweeps, the stores.  Launches are chained (grid_wait):
-// the tile's constants (positions, parameters, rest Darboux, inertial targets) are loaded while the iteration
-// before still runs.  256,000 vertices, 20 iterations, the whole tied step: 211 us with ordinary launches, 190.
-__global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, const float4* __restrict__ y4, float4* q,
+// the tile's constants (positions, parameters, rest Darboux) are loaded while the launch before still runs.  256,000 vertices, 20 iterations, the whole tied step: 211 us with ordinary launches, 190.
+__global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, const float4* y4, float4* q,
                                                               const float4* dx_in,
                                                               float4* __restrict__ dx_out,
                                                               const StepParams* __restrict__ spp, PhysParams pp, int C) {
@@ -185,7 +186,6 @@ __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, co
         sx[p] = st.xm[g];
         sprm[p] = st.prm[g];
         sqr[p] = st.qr[g];
-        yown[c] = xyz(y4[g]);
     }
     const float h = spp->h;
     const float damp = pp.damping / h;
@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, co
 #pragma unroll
     for (int c = 0; c < 2; c++) {
         const int p = (row2 + c) * 32 + lane;
+        yown[c] = xyz(load_fresh(y4 + base + p));
         sdx[p] = load_fresh(dx_in + base + p);
         sq[p] = load_fresh(q + base + p);
     }
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, co
 // previous orientations (double-buffered in shared memory), as the two Jacobi launches
 // (sweep_position_kernel<true>, sweep_orientation_kernel<true>) do.  Tied partners' dx come from
 // dx_in, the previous iterate.  dx goes to dx_out, q to q_out.
-__global__ void __launch_bounds__(512) sweep_iteration_jacobi_kernel(DeviceState st, const float4* __restrict__ y4,
+__global__ void __launch_bounds__(512) sweep_iteration_jacobi_kernel(DeviceState st, const float4* y4,
                                                                      const float4* q_in,
                                                                      float4* __restrict__ q_out,
                                                                      const float4* dx_in,
@@ -305,7 +306,6 @@ __global__ void __launch_bounds__(512) sweep_iteration_jacobi_kernel(DeviceState
         sx[p] = st.xm[g];
         sprm[p] = st.prm[g];
         sqr[p] = st.qr[g];
-        yown[c] = xyz(y4[g]);
     }
     const float h = spp->h;
     const float damp = pp.damping / h;
@@ -314,6 +314,7 @@ __global__ void __launch_bounds__(512) sweep_iteration_jacobi_kernel(DeviceState
 #pragma unroll
     for (int c = 0; c < 2; c++) {
         const int p = (row2 + c) * 32 + lane;
+        yown[c] = xyz(load_fresh(y4 + base + p));
         sdx[p] = load_fresh(dx_in + base + p);
         sq[p] = load_fresh(q_in + base + p);
     }
@@ -426,9 +427,11 @@ cudaError_t launch_sweep_iteration(const DeviceState& st, const float4* y4, cons
 }
 
 // endItr for every slot, then (on the last substep) the SDF pass and the finiteness check.
-__global__ void sweep_finish_kernel(DeviceState st, const float4* __restrict__ dx4, const StepParams* __restrict__ spp,
+__global__ void sweep_finish_kernel(DeviceState st, const float4* dx4, const StepParams* __restrict__ spp,
                                     PhysParams pp, SdfParams sdf, int apply_sdf, int64_t num_slots) {
     int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    grid_wait();
+    grid_release();
     bool bad = false;
     if (g < num_slots) {
         const StepParams sp = *spp;
@@ -575,9 +578,9 @@ __global__ void gather_slots_kernel(const float4* __restrict__ src, float* __res
 static inline unsigned blocks_for(int64_t n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
 cudaError_t launch_sweep_predict(const DeviceState& st, float4* y4, float4* dx4, const StepParams* d_sp,
-                                 const PhysParams& pp, int64_t num_slots, cudaStream_t s) {
-    sweep_predict_kernel<<<blocks_for(num_slots, 256), 256, 0, s>>>(st, y4, dx4, d_sp, pp, num_slots);
-    return cudaGetLastError();
+                                 const PhysParams& pp, int64_t num_slots, bool chained, cudaStream_t s) {
+    return launch_chained(chained, sweep_predict_kernel, blocks_for(num_slots, 256), 256, 0, s, st, y4, dx4, d_sp, pp,
+                          num_slots);
 }
 
 cudaError_t launch_sweep_position(const DeviceState& st, const float4* y4, const float4* q, const float4* dx_in,
@@ -605,9 +608,9 @@ cudaError_t launch_sweep_orientation(const DeviceState& st, const float4* dx4, c
 }
 
 cudaError_t launch_sweep_finish(const DeviceState& st, const float4* dx4, const StepParams* d_sp, const PhysParams& pp,
-                                const SdfParams& sdf, bool apply_sdf, int64_t num_slots, cudaStream_t s) {
-    sweep_finish_kernel<<<blocks_for(num_slots, 256), 256, 0, s>>>(st, dx4, d_sp, pp, sdf, apply_sdf ? 1 : 0, num_slots);
-    return cudaGetLastError();
+                                const SdfParams& sdf, bool apply_sdf, int64_t num_slots, bool chained, cudaStream_t s) {
+    return launch_chained(chained, sweep_finish_kernel, blocks_for(num_slots, 256), 256, 0, s, st, dx4, d_sp, pp, sdf,
+                          apply_sdf ? 1 : 0, num_slots);
 }
 
 // SDFBodyCollisionSolver's StrainLimiting (SDFCollisionSolver/cudaSDFCollision.cu:176-199): one

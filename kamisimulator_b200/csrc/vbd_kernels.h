@@ -26,7 +26,7 @@ cudaError_t launch_chained(bool chained, void (*kernel)(P...), unsigned grid, un
 }
 
 cudaError_t launch_sweep_predict(const DeviceState& st, float4* y4, float4* dx4, const StepParams* d_sp,
-                                 const PhysParams& pp, int64_t num_slots, cudaStream_t s);
+                                 const PhysParams& pp, int64_t num_slots, bool chained, cudaStream_t s);
 // conn_dx: the partners' dx for tied vertices (st.conn), the iteration's starting values
 cudaError_t launch_sweep_position(const DeviceState& st, const float4* y4, const float4* q, const float4* dx_in,
                                   float4* dx_out, const StepParams* d_sp, const PhysParams& pp, int C, int colour,
@@ -34,7 +34,6 @@ cudaError_t launch_sweep_position(const DeviceState& st, const float4* y4, const
 // One iteration (colour2: both position sweeps, both orientation sweeps; jacobi: the position and
 // the orientation sweep) in one launch, one block per tile of up to 1024 slots: reads dx_in, writes
 // dx_out; q in place for colour2 (q_in == q_out), into q_out for jacobi (sweep_iteration_supported).
-// chained: only behind another iteration of the same substep (it reads y4 ahead of grid_wait).
 bool sweep_iteration_supported(int C);
 cudaError_t launch_sweep_iteration(const DeviceState& st, const float4* y4, const float4* q_in, float4* q_out,
                                    const float4* dx_in, float4* dx_out, const StepParams* d_sp, const PhysParams& pp,
@@ -42,7 +41,7 @@ cudaError_t launch_sweep_iteration(const DeviceState& st, const float4* y4, cons
 cudaError_t launch_sweep_orientation(const DeviceState& st, const float4* dx4, const float4* q_in, float4* q_out, int C,
                                      int colour, bool jacobi, cudaStream_t s);
 cudaError_t launch_sweep_finish(const DeviceState& st, const float4* dx4, const StepParams* d_sp, const PhysParams& pp,
-                                const SdfParams& sdf, bool apply_sdf, int64_t num_slots, cudaStream_t s);
+                                const SdfParams& sdf, bool apply_sdf, int64_t num_slots, bool chained, cudaStream_t s);
 
 bool fused_supported(int C);
 // nsteps consecutive steps in one launch: parameters from d_steps[0..nsteps) (device), or sp when
@@ -72,13 +71,16 @@ cudaError_t launch_adjoint_step(const DeviceState& st, const PhysParams& pp, con
 // bucket scan of a table of n buckets needs.
 int64_t coll_scan_tmp_size(int64_t n);
 cudaError_t launch_coll_detect(const DeviceState& st, const float4* dx4, const CollParams& cp, cudaStream_t s);
-cudaError_t launch_coll_steplimit(const DeviceState& st, const float4* dx4, const CollParams& cp, cudaStream_t s);
+cudaError_t launch_coll_steplimit(const DeviceState& st, const float4* dx4, const CollParams& cp, bool chained,
+                                  cudaStream_t s);
 // One colour2 iteration of the sweep form with contacts in one launch (one block per tile, one
 // thread per slot): reads the iteration's starting displacements from snap, writes dx_out, updates
-// q in place.  Tiles of up to 1024 slots (coll_iteration_supported).
+// q in place.  Tiles of up to 1024 slots (coll_iteration_supported).  chained: only behind another iteration of
+// the same substep (it reads y4 and the contact lists ahead of grid_wait).
 bool coll_iteration_supported(int C);
 cudaError_t launch_coll_iteration(const DeviceState& st, const float4* y4, float4* q, const float4* snap, float4* dx_out,
-                                  const StepParams* d_sp, const PhysParams& pp, const CollParams& cp, bool chained, cudaStream_t s);
+                                  const StepParams* d_sp, const PhysParams& pp, const CollParams& cp, bool chained,
+                                  cudaStream_t s);
 cudaError_t launch_sweep_position_coll(const DeviceState& st, const float4* y4, const float4* q, const float4* dx_in,
                                        float4* dx_out, const float4* snap, const StepParams* d_sp, const PhysParams& pp,
                                        const CollParams& cp, int colour, bool jacobi, cudaStream_t s);
