@@ -95,10 +95,10 @@ __device__ __forceinline__ float4 fused_orientation(float4 q, bool upd, bool pre
     return upd ? n : q;
 }
 
-template <int C, bool GROUPED>
+template <int C, bool GROUPED, bool RECORD = true>
 __device__ __forceinline__ void recorded_step_body(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf, TapeView tp,
                                                    const StepParams* __restrict__ steps, int nsteps) {
-    constexpr bool RECORD = true;  // (one step of one substep: the launch's steps / nsteps are null and 1)
+    // (RECORD: one step of one substep, the launch's steps / nsteps are null and 1)
     const int lane = threadIdx.x & 31;
     const int64_t tile = (RECORD ? tp.tile_begin : 0) + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (tile >= st.num_tiles) return;  // uniform per warp (per CTA for groups: num_tiles is a multiple of K)
@@ -333,6 +333,12 @@ template <int C>
 __global__ void __launch_bounds__(256) recorded_group_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
                                                              TapeView tp) {
     recorded_step_body<C, true>(st, pp, sp, sdf, tp, nullptr, 1);
+}
+// The same without a tape: the plain step of few groups (launch_scalar_group).
+template <int C>
+__global__ void __launch_bounds__(256) scalar_group_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
+                                                           const StepParams* __restrict__ steps, int nsteps) {
+    recorded_step_body<C, true, false>(st, pp, sp, sdf, TapeView{}, steps, nsteps);
 }
 
 __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
@@ -866,6 +872,18 @@ __global__ void __launch_bounds__(NT, MINB) adjoint_step_kernel(DeviceState st, 
 }
 
 // ------------------------------------------------------------------------------------------
+cudaError_t launch_scalar_group(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
+                                int C, int group, cudaStream_t s, const StepParams* d_steps, int nsteps) {
+    if (group < 1 || group > 8 || st.num_tiles % group != 0 || (C != 2 && C != 4)) return cudaErrorInvalidValue;
+    const unsigned blocks = (unsigned)(st.num_tiles / group);
+    if (blocks == 0) return cudaSuccess;
+    if (C == 2)
+        scalar_group_kernel<2><<<blocks, 32 * group, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);
+    else
+        scalar_group_kernel<4><<<blocks, 32 * group, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_fused_record(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
                                 const TapeView& tp, int C, int warps_per_block, cudaStream_t s, int group) {
     if (group > 1) {  // one CTA of `group` warps per group of tiles (the window is whole groups)

@@ -839,6 +839,15 @@ cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const
         const unsigned gblocks = (unsigned)(st.num_tiles / group);
         if (gblocks == 0) return cudaSuccess;
         const int gthreads = 32 * group;
+        // Up to one warp a scheduler (4 an SM) a group's time is its chain of dependent instructions, and the
+        // paired ones, with the moves between their layouts, make the colour2 chain longer: 42 substeps of 32
+        // iterations take 815 us in scalar FP32 and 873 paired at 480 tiles.  With more tiles the schedulers
+        // share issue slots: 1317 against 1258 us at 652 tiles, 10.9 ms against 10.35 at 9,600.  Jacobi: paired
+        // at every size (828 against 767 us at 480 tiles).
+        int dev = 0, sms = 0;
+        if (!jacobi && reg_cap <= 1 && cudaGetDevice(&dev) == cudaSuccess &&
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && st.num_tiles <= 4LL * sms)
+            return launch_scalar_group(st, pp, sp, sdf, C, group, s, d_steps, nsteps);
 #define KAMI_GROUP_LAUNCH(KERNEL, CC)                                                                   \
     do {                                                                                                \
         if (jacobi)                                                                                     \

@@ -137,3 +137,35 @@ def test_nonfinite_long_strand_does_not_leak(slots):
     assert not np.isfinite(xb[a:b]).all()
     clean.close()
     bad.close()
+
+
+@pytest.mark.parametrize("length", [129, 256, 300])
+def test_taped_handle_steps_long_strands_as_it_records_them(length):
+    """A handle with a tape steps groups of tiles with the recording kernel: the checkpoints of a rollout and its
+    recomputed segments are the same numbers, bit for bit."""
+    g = helpers.soft_groom(3, (length, length), seed=length)
+    s = helpers.gpu_solver(g, helpers.soft_settings(num_itr=4), form="fused")
+    try:
+        start = s.get_state()
+        s.tape_reserve(2, 0)
+        for _ in range(2):
+            s.step(1 / 60)
+        plain = s.get_state()
+        s.set_state(start)
+        for _ in range(2):
+            s.step_record(1 / 60)
+        recorded = s.get_state()
+    finally:
+        s.close()
+    assert not np.array_equal(plain, start)
+    np.testing.assert_array_equal(plain, recorded)
+
+
+@pytest.mark.parametrize("strands", [1, 147, 148, 149, 297])
+def test_few_and_many_groups_match_the_oracle(strands):
+    """Groups of 4 tiles on both sides of the size at which the colour2 step changes kernels (4 tiles an SM).  The
+    bar is that of one step: FP32 rounding of 0.1 m coordinates and num_itr corrections, well below it."""
+    g = helpers.soft_groom(strands, (400, 400), seed=strands)
+    s = helpers.soft_settings(num_itr=4, max_h=1 / 120, sdf=synth.sphere_sdf(32, radius=0.09, half_extent=0.6))
+    ex, et = _lockstep(g, s, "fused", 1, 1 / 60)
+    assert ex <= 1e-5 and et <= 1e-5, (ex, et)

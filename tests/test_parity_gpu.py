@@ -284,3 +284,68 @@ def test_stepping_calls_check_dt():
     with pytest.raises(KamiError, match="INVALID_ARGUMENT"):
         s.set_launch_mode(7)
     s.close()
+
+
+@pytest.mark.parametrize("schedule", ["colour2", "jacobi"])
+@pytest.mark.parametrize("slots", [2, 4])
+@pytest.mark.parametrize("length", [3, 31, 32, 33, 63, 64])
+def test_packed_step_at_tile_edges(length, slots, schedule):
+    """Strands that start, end and meet at every place of a lane, a row and a tile (64 or 128 slots), an odd
+    number of them, with the SDF pass and two substeps.  A step's positions are sums of a few 0.1 m terms in
+    FP32 (2e-8 m each) and at most num_itr corrections of the same size, well inside the bar of one step."""
+    g = helpers.soft_groom(37, (length, length), seed=length)
+    sdf = synth.sphere_sdf(32, radius=0.09, half_extent=0.3, threshold=2e-3)
+    st = helpers.soft_settings(schedule=schedule, max_h=1 / 120, num_itr=5, sdf=sdf, wind=(2.0, 1.0, 0.7, 0.4, 3.0),
+                               slots_per_lane=slots)
+    v = helpers.random_velocities(g, 0.2, seed=2)
+    ost = {k: a for k, a in st.items() if k != "slots_per_lane"}
+    o = helpers.oracle_sim(g, ost, np.float32, v)
+    s = helpers.gpu_solver(g, st, form="fused", velocities=v)
+    try:
+        o.advance(1 / 60)
+        s.step(1 / 60)
+        x, _ = s.get_positions_velocities()
+        q = s.get_orientations()
+    finally:
+        s.close()
+    assert np.abs(x - o.x).max() <= POS_TOL
+    assert np.abs(twist_angles(o.q, q)).max() <= TWIST_TOL
+
+
+@pytest.mark.parametrize("strands,length", [(1, 3), (85, 3), (129, 64)])
+@pytest.mark.parametrize("skew", [0, 1])
+def test_device_boundary_arrays_equal_the_host_ones(skew, strands, length):
+    """Reads and writes of one or two arrays, a state and orientations in device memory (skew: arrays that start
+    4 bytes past an allocation) against the same through host memory: copies, so bit for bit."""
+    import torch
+
+    g = helpers.soft_groom(strands, (length, length), seed=5)
+    s = helpers.gpu_solver(g, helpers.soft_settings(num_itr=3), velocities=helpers.random_velocities(g))
+    nv = s.num_vertices
+
+    def dev(n):
+        return torch.full((n + skew,), -7.0, device="cuda")[skew:]
+
+    try:
+        s.step(1 / 60)
+        x, v = s.get_positions_velocities()
+        q, state = s.get_orientations(), s.get_state()
+        dx, dv, dq, ds = dev(3 * nv), dev(3 * nv), dev(4 * nv), dev(state.size)
+        s.get_positions_velocities(dx, dv)
+        s.get_orientations(dq)
+        s.get_state_into(ds)
+        for a, b in ((dx, x), (dv, v), (dq, q), (ds, state)):
+            np.testing.assert_array_equal(a.cpu().numpy().view(np.int32), b.ravel().view(np.int32))
+        only_v = dev(3 * nv)
+        s.get_positions_velocities(None, only_v)
+        np.testing.assert_array_equal(only_v.cpu().numpy(), v.ravel())
+        s.set_positions_velocities(dx + 1.0, None)
+        s.set_positions_velocities(None, 2.0 * dv)
+        x2, v2 = s.get_positions_velocities()
+        np.testing.assert_array_equal(x2.ravel(), x.ravel() + np.float32(1.0))
+        np.testing.assert_array_equal(v2.ravel(), 2 * v.ravel())
+        s.step(1 / 60)
+        s.set_state_from(ds)
+        np.testing.assert_array_equal(s.get_state().view(np.int32), state.view(np.int32))
+    finally:
+        s.close()
