@@ -215,10 +215,11 @@ __host__ __device__ __forceinline__ float3 qrotate(float4 r, float3 v) {
 
 // Chained launches (programmatic dependent launch): a kernel launched with launch_chained may start before
 // the kernel ahead of it in the stream has ended.  grid_wait() returns when that one is complete and its
-// writes are visible; before it, only what no kernel still running can write may be read.  Every kernel of
-// such a chain calls both, grid_wait first, so at most two of its kernels are in flight and what was complete
-// before the kernel ahead passed its own grid_wait is safe to read at once.  Both do nothing in a kernel
-// launched the ordinary way.
+// writes are visible.  Ahead of it a kernel may only read what was complete before the latest ordinary launch
+// of the stream began: that launch made it visible, and nothing in flight writes it.  (That an earlier kernel
+// of the chain has ended is not enough: only grid_wait makes its writes visible to the grid that waits, and
+// an older value may still lie in L1.)  Every kernel of a chain calls both, grid_wait first, so at most two
+// of its kernels are in flight.  Both do nothing in a kernel launched the ordinary way.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // A read that stays behind grid_wait (volatile) and sees other SMs' writes (L2).

@@ -164,7 +164,9 @@ __global__ void sweep_orientation_kernel(DeviceState st, const float4* __restric
 // the state is read once per iteration instead of once per sweep.  dx goes to dx_out, q is updated
 // in place.
 // Bound by latency: a launch, the loads, four dependent sweeps, the stores.  Launches are chained (grid_wait):
-// the tile's constants (positions, parameters, rest Darboux) are loaded while the launch before still runs.  256,000 vertices, 20 iterations, the whole tied step: 211 us with ordinary launches, 190.
+// the tile's constants (positions, parameters, rest Darboux) are loaded while the launch before still runs.
+// A substep's first iteration is an ordinary launch, since the finish of the substep before wrote the positions.
+// 256,000 vertices, 20 iterations, the whole tied step: 211 us with ordinary launches, 190.
 __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, const float4* y4, float4* q,
                                                               const float4* dx_in,
                                                               float4* __restrict__ dx_out,
