@@ -1065,26 +1065,7 @@ kami_status kami_vbd_step(kami_vbd_handle h, float dt, void* stream) {
     const StepParams sp = advance_clock(h, dt);
     const int steps = sp.substeps;
     kami_status st = on_stream(h, stream, [&](cudaStream_t s) -> kami_status {
-        if (h->form == KAMI_FORM_FUSED && h->tape_capacity > 0 && h->layout.K > 1) {
-            // groups of tiles on a handle with a tape (colour2): the plain step rounds differently there, and a
-            // segment recomputed from a checkpoint has to repeat the steps that led there to the bit, so
-            // these steps are recorded too, over and over into one row of scratch (the adjoint's
-            // buffers, which hold nothing between two backward calls)
-            StepParams sp1 = sp;
-            sp1.substeps = 1;
-            SdfParams no_sdf = h->sdf;
-            no_sdf.grid = nullptr;
-            TapeView row{};
-            row.dx = row.vl = h->d_gx;
-            row.q = h->d_gq;
-            row.x = h->d_gv;
-            row.v = h->d_gvl;
-            row.num_itr = h->pp.num_itr;
-            for (int k = 0; k < steps; k++)
-                KAMI_CUDA(launch_fused_record(h->dstate(), h->pp, sp1, k == steps - 1 ? h->sdf : no_sdf, row, h->layout.C,
-                                              h->warps_per_block, s, h->layout.K),
-                          "recorded step launch");
-        } else if (h->form == KAMI_FORM_FUSED) {
+        if (h->form == KAMI_FORM_FUSED) {
             KAMI_CUDA(launch_fused_step(h->dstate(), h->pp, sp, h->sdf, h->layout.C, h->schedule == KAMI_SCHEDULE_JACOBI,
                                         h->warps_per_block, s, nullptr, 1, h->reg_cap, h->layout.K, h->launch_mode),
                       "fused step launch");

@@ -1,8 +1,8 @@
 // vbd_adjoint.cu -- reverse-mode adjoint of the fused colour2 VBD step (one substep per step).
 //
-// The forward step is recorded by recorded_step_kernel<C>: the start state and, after the predict
-// and after every iteration, every slot's displacement iterate dx and segment orientation q.  adjoint_step_kernel<C> walks one recorded step backwards, one warp per
-// tile as in the forward:
+// The forward step is recorded by recorded_step_kernel<C> (vbd_scalar.cuh): the start state and, after the
+// predict and after every iteration, every slot's displacement iterate dx and segment orientation q.
+// adjoint_step_kernel<C> walks one recorded step backwards, one warp per tile as in the forward:
 //
 //   SDF pass  ->  velocity update  ->  iterations N..1, each as
 //     orientation sweep odd segments, even segments, position sweep odd vertices, even vertices
@@ -21,7 +21,7 @@
 // through the inertial target and the initial guess (iteration.cu:8-59), and with wind the start
 // position's y and z through the wind force in both.  The parameter gradient
 // d loss / d qRest accumulates in AdjointState::gqr.
-#include "vbd_fused.cuh"
+#include "vbd_scalar.cuh"
 #include "vbd_kernels.h"
 
 namespace kami {
@@ -35,311 +35,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all_but_one() { asm volatile("cp.async.wait_group 1;\n" ::: "memory"); }
-// ---- recorded steps ----------------------------------------------------------------------------------
-// The forward step that the tape holds, with scalar updates that orientation_adjoint below reverses as they
-// round: a stiffness gradient sits on the kinks of the predict's clamp and of the body pass, and with
-// another rounding of the same step it moves by 1e-5 to 1e-4 of itself.
-__device__ __forceinline__ float sqrt_nonneg(float x) { return x * rsqrt_ftz(fmaxf(x, 1e-30f)); }
-// One position update with folded coefficients (see the file comment).  Neighbour operands from
-// another strand (no segment in between: hn / hp false) are replaced by the vertex's own values
-// before they meet their zero coefficient, and vertices that do not move (upd false) keep dx, so a
-// non-finite strand cannot leak into the strands or padding that share its tile, as the
-// reference's flag tests guarantee.  Strands start at even tile positions, so only the previous
-// neighbour of an even slot and the next neighbour of an odd slot can belong to another strand;
-// the others are the same strand or padding (always finite), and guard_next / guard_prev say
-// which operands need the replacement (the results are the same bit for bit either way).  Padding
-// and pinned slots keep their dx through the final select: padding must stay finite, as the
-// strand before it reads it unguarded and a restored state does not rewrite padding.
-__device__ __forceinline__ float3 fused_position(float3 dx, float3 F0, float ddN, float kkN, float3 d3N, float3 dxN,
-                                                 float ddP, float kkP, float3 d3P, float3 dxP, float as_, float isA,
-                                                 float isD, bool hn, bool hp, bool upd, bool guard_next,
-                                                 bool guard_prev) {
-    if (guard_next) dxN = hn ? dxN : dx;
-    if (guard_prev) {
-        dxP = hp ? dxP : dx;
-        d3P = hp ? d3P : d3N;
-    }
-    float3 f;
-    f.x = F0.x + ddN * dxN.x + ddP * dxP.x - as_ * dx.x - kkN * d3N.x + kkP * d3P.x;
-    f.y = F0.y + ddN * dxN.y + ddP * dxP.y - as_ * dx.y - kkN * d3N.y + kkP * d3P.y;
-    f.z = F0.z + ddN * dxN.z + ddP * dxP.z - as_ * dx.z - kkN * d3N.z + kkP * d3P.z;
-    const float m = (f.x + f.y + f.z) * (1.f / 3.f);
-    const float3 n = f3(fmaf(m, isD, fmaf(f.x, isA, dx.x)), fmaf(m, isD, fmaf(f.y, isA, dx.y)),
-                        fmaf(m, isD, fmaf(f.z, isA, dx.z)));
-    return upd ? n : dx;
-}
-
-// One orientation update (quaternionLambdaItr), branch-free: pre/nxt say whether the previous /
-// next segment exists, upd whether this segment is updated at all; guard_prev / guard_next as in
-// fused_position.
-__device__ __forceinline__ float4 fused_orientation(float4 q, bool upd, bool pre, bool nxt, float3 Ve, float m2k,
-                                                    float3 dx, float3 dxN, float4 qPrev, float4 qrPrev, float4 qNext,
-                                                    float4 qr, bool guard_prev, bool guard_next) {
-    const float3 V = Ve + m2k * (dxN - dx);
-    if (guard_prev) qPrev = pre ? qPrev : q;  // operands from another strand never meet arithmetic
-    if (guard_next) qNext = nxt ? qNext : q;
-    const float4 P1 = qmul_fma(qPrev, qrPrev);
-    const float4 P2 = qmul_conj_fma(qNext, qr);
-    float s1 = dot4(q, P1) > 0.f ? 1.f : -1.f;
-    float s2 = dot4(q, P2) > 0.f ? 1.f : -1.f;
-    s1 = pre ? s1 : 0.f;
-    s2 = nxt ? s2 : 0.f;
-    const float4 b = make_float4(s1 * P1.x + s2 * P2.x, s1 * P1.y + s2 * P2.y, s1 * P1.z + s2 * P2.z,
-                                 s1 * P1.w + s2 * P2.w);
-    const float lambda = sqrt_nonneg(dot3(V, V)) + sqrt_nonneg(dot4(b, b));
-    const float3 bq = f3(b.x, b.y, b.z);
-    const float3 Pq = b.w * V + cross3(V, bq);
-    const float Pw = -dot3(V, bq);
-    const float4 R = make_float4(Pw + lambda * b.x, Pq.z + lambda * b.y, -Pq.y + lambda * b.z, -Pq.x + lambda * b.w);
-    const float4 n = scale4(rsqrt_ftz(dot4(R, R)), R);
-    return upd ? n : q;
-}
-
-template <int C, bool GROUPED, bool RECORD = true>
-__device__ __forceinline__ void recorded_step_body(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf, TapeView tp,
-                                                   const StepParams* __restrict__ steps, int nsteps) {
-    // (RECORD: one step of one substep, the launch's steps / nsteps are null and 1)
-    const int lane = threadIdx.x & 31;
-    const int64_t tile = (RECORD ? tp.tile_begin : 0) + (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (tile >= st.num_tiles) return;  // uniform per warp (per CTA for groups: num_tiles is a multiple of K)
-    const int64_t base = tile * (32LL * C) + lane;
-    // tile groups: neighbours across the warps of the CTA (see GroupExchange)
-    const int gw = threadIdx.x >> 5, gK = blockDim.x >> 5;
-    GroupExchange* gx = nullptr;
-    if constexpr (GROUPED) {
-        __shared__ GroupExchange group_exchange;
-        gx = &group_exchange;
-    }
-    auto up_put = [&](int slot, float4 v) {
-        if (GROUPED && lane == 31) gx->up[gw][slot] = v;
-    };
-    auto up_get = [&](int slot, float4 v) { return (GROUPED && lane == 0 && gw > 0) ? gx->up[gw - 1][slot] : v; };
-    auto down_put = [&](int slot, float4 v) {
-        if (GROUPED && lane == 0) gx->down[gw][slot] = v;
-    };
-    auto down_get = [&](int slot, float4 v) { return (GROUPED && lane == 31 && gw < gK - 1) ? gx->down[gw + 1][slot] : v; };
-    auto group_sync = [&]() {
-        if (GROUPED) __syncthreads();
-    };
-    auto f4 = [](float3 a) { return make_float4(a.x, a.y, a.z, 0.f); };
-
-    float3 x[C], v[C], vl[C], dx[C], d3[C], F0[C], Ve[C];
-    float4 q[C], qr[C];
-    float im[C], invl[C], kk[C], ddN[C], kkN[C], as_[C], isA[C], isD[C];
-    uint32_t fl[C];
-    bool mov[C];  // the vertex's position is updated (not pinned, not padding)
-
-#pragma unroll
-    for (int k = 0; k < C; k++) {
-        const int64_t g = base + 32LL * k;
-        const float4 a = st.xm[g];
-        x[k] = xyz(a);
-        im[k] = a.w;
-        v[k] = xyz(st.vel[g]);
-        vl[k] = xyz(st.vlast[g]);
-        q[k] = st.q[g];
-        qr[k] = st.qr[g];
-        const float4 p = st.prm[g];
-        invl[k] = 1.f / p.x;
-        kk[k] = p.y * invl[k];
-        fl[k] = __float_as_uint(p.w);
-        mov[k] = im[k] != 0.f;
-        ddN[k] = (fl[k] & F_HAS_NEXT) ? kk[k] * invl[k] : 0.f;
-        kkN[k] = (fl[k] & F_HAS_NEXT) ? kk[k] : 0.f;
-    }
-    const int64_t tS = tp.slots;
-    const int64_t tslot = base - (RECORD ? tp.tile_begin * 32LL * C : 0);  // this lane's slot in the tape window
-    const int64_t tbase = ((int64_t)tp.step * (tp.num_itr + 1)) * tS + tslot;  // tape row of iteration 0
-    if (RECORD) {
-#pragma unroll
-        for (int k = 0; k < C; k++) {
-            const int64_t o = (int64_t)tp.step * tS + tslot + 32LL * k;
-            tp.x[o] = make_float4(x[k].x, x[k].y, x[k].z, im[k]);
-            tp.v[o] = make_float4(v[k].x, v[k].y, v[k].z, 0.f);
-            tp.vl[o] = make_float4(vl[k].x, vl[k].y, vl[k].z, 0.f);
-        }
-    }
-    // constants of the previous lane's last segment (segment i-1 of slot 0)
-    float4 qrH = shfl_up4(qr[C - 1], 1);
-    float ddH = __shfl_up_sync(0xffffffffu, ddN[C - 1], 1);
-    float kkH = __shfl_up_sync(0xffffffffu, kkN[C - 1], 1);
-    if (GROUPED) {
-        up_put(XU_QR, qr[C - 1]);
-        up_put(XU_DK, make_float4(ddN[C - 1], kkN[C - 1], 0.f, 0.f));
-        group_sync();
-        qrH = up_get(XU_QR, qrH);
-        const float4 dk = up_get(XU_DK, make_float4(ddH, kkH, 0.f, 0.f));
-        ddH = dk.x;
-        kkH = dk.y;
-    }
-
-    const float accel = pp.accel_ratio;
-    bool bad = false;
-    for (int step = 0; step < nsteps; step++) {
-    if (steps) sp = steps[step];
-    const float h = sp.h;
-    const float damp = pp.damping / h;
-
-    for (int s = 0; s < sp.substeps; s++) {
-        {
-            float3 e[C];
-#pragma unroll
-            for (int k = 0; k < C - 1; k++) e[k] = x[k + 1] - x[k];
-            float3 xN0 = shfl_down3(x[0], 1);
-            if (GROUPED) {
-                down_put(XD_X, f4(x[0]));
-                group_sync();
-                xN0 = xyz(down_get(XD_X, f4(xN0)));
-            }
-            e[C - 1] = xN0 - x[C - 1];
-#pragma unroll
-            for (int k = 0; k < C; k++) e[k] = (fl[k] & F_HAS_NEXT) ? e[k] : f3(0.f, 0.f, 0.f);
-            float3 eH = shfl_up3(e[C - 1], 1);
-            if (GROUPED) {
-                up_put(XU_E, f4(e[C - 1]));
-                group_sync();
-                eH = xyz(up_get(XU_E, f4(eH)));
-            }
-#pragma unroll
-            for (int k = 0; k < C; k++) {
-                float3 y;
-                vbd_predict(x[k], v[k], vl[k], im[k], pp, h, sp.last_h, sp.time, dx[k], y);
-                vl[k] = v[k];
-                const float ddP = k > 0 ? ddN[k > 0 ? k - 1 : 0] : ddH;
-                const float3 eP = k > 0 ? e[k > 0 ? k - 1 : 0] : eH;
-                const float a = im[k] != 0.f ? 1.f / (im[k] * h * h) : 0.f;
-                const float sk = (ddN[k] + ddP) * (1.f + damp);
-                as_[k] = a + sk;
-                isA[k] = im[k] != 0.f ? accel / sk : 0.f;
-                isD[k] = im[k] != 0.f ? accel / (sk + 3.f * a) - isA[k] : 0.f;
-                F0[k] = a * y + ddN[k] * e[k] - ddP * eP;
-                Ve[k] = (-2.f * kk[k]) * e[k];
-                d3[k] = d3_of(q[k]);
-            }
-        }
-        float4 qP = shfl_up4(q[C - 1], 1);
-        float3 d3P = shfl_up3(d3[C - 1], 1);  // the previous lane's d3_of(qP)
-        if (RECORD) {
-#pragma unroll
-            for (int k = 0; k < C; k++) {
-                tp.dx[tbase + 32LL * k] = make_float4(dx[k].x, dx[k].y, dx[k].z, 0.f);
-                tp.q[tbase + 32LL * k] = q[k];
-            }
-        }
-
-        for (int it = 0; it < pp.num_itr; it++) {
-            {
-                float3 dxP = shfl_up3(dx[C - 1], 1);
-                if (GROUPED) {  // the previous lane's odd values, unchanged until the odd sweeps
-                    up_put(XU_DX, f4(dx[C - 1]));
-                    up_put(XU_Q, q[C - 1]);
-                    up_put(XU_D3, f4(d3[C - 1]));
-                    group_sync();
-                    dxP = xyz(up_get(XU_DX, f4(dxP)));
-                    qP = up_get(XU_Q, qP);
-                    d3P = xyz(up_get(XU_D3, f4(d3P)));
-                }
-                // positions, even slots (neighbours are odd: own registers or the previous lane)
-                {
-#pragma unroll
-                    for (int k = 0; k < C; k += 2) {
-                        const int kp = k > 0 ? k - 1 : 0;
-                        dx[k] = fused_position(dx[k], F0[k], ddN[k], kkN[k], d3[k], dx[k + 1], k ? ddN[kp] : ddH,
-                                               k ? kkN[kp] : kkH, k ? d3[kp] : d3P, k ? dx[kp] : dxP, as_[k], isA[k],
-                                               isD[k], fl[k] & F_HAS_NEXT, fl[k] & F_HAS_PREV, mov[k], false, true);
-                    }
-                }
-                // positions, odd slots
-                float3 dxN0 = shfl_down3(dx[0], 1);
-                if (GROUPED) {
-                    down_put(XD_DX, f4(dx[0]));
-                    group_sync();
-                    dxN0 = xyz(down_get(XD_DX, f4(dxN0)));
-                }
-#pragma unroll
-                for (int k = 1; k < C; k += 2) {
-                    const int kn = k + 1 < C ? k + 1 : k;
-                    dx[k] = fused_position(dx[k], F0[k], ddN[k], kkN[k], d3[k], k == C - 1 ? dxN0 : dx[kn], ddN[k - 1],
-                                           kkN[k - 1], d3[k - 1], dx[k - 1], as_[k], isA[k], isD[k],
-                                           fl[k] & F_HAS_NEXT, fl[k] & F_HAS_PREV, mov[k], true, false);
-                }
-                // orientations, even segments
-#pragma unroll
-                for (int k = 0; k < C; k += 2) {
-                    const int kp = k > 0 ? k - 1 : 0;
-                    const uint32_t f = fl[k];
-                    q[k] = fused_orientation(q[k], (f & F_HAS_NEXT) && !(f & F_FIX_ORIENTATION), f & F_HAS_PREV,
-                                             f & F_HAS_NEXT_ORIENTATION, Ve[k], -2.f * kk[k], dx[k], dx[k + 1],
-                                             k ? q[kp] : qP, k ? qr[kp] : qrH, q[k + 1], qr[k], true, false);
-                    d3[k] = d3_of(q[k]);
-                }
-                // orientations, odd segments
-                float4 qN0 = shfl_down4(q[0], 1);
-                if (GROUPED) {
-                    down_put(XD_Q, q[0]);
-                    group_sync();
-                    qN0 = down_get(XD_Q, qN0);
-                }
-#pragma unroll
-                for (int k = 1; k < C; k += 2) {
-                    const int kn = k + 1 < C ? k + 1 : k;
-                    const uint32_t f = fl[k];
-                    q[k] = fused_orientation(q[k], (f & F_HAS_NEXT) && !(f & F_FIX_ORIENTATION), f & F_HAS_PREV,
-                                             f & F_HAS_NEXT_ORIENTATION, Ve[k], -2.f * kk[k], dx[k],
-                                             k == C - 1 ? dxN0 : dx[kn], q[k - 1], qr[k - 1],
-                                             k == C - 1 ? qN0 : q[kn], qr[k], false, true);
-                    d3[k] = d3_of(q[k]);
-                }
-                qP = shfl_up4(q[C - 1], 1);
-                d3P = shfl_up3(d3[C - 1], 1);
-                if (RECORD) {
-                    const int64_t row = tbase + (int64_t)(it + 1) * tS;
-#pragma unroll
-                    for (int k = 0; k < C; k++) {
-                        tp.dx[row + 32LL * k] = make_float4(dx[k].x, dx[k].y, dx[k].z, 0.f);
-                        tp.q[row + 32LL * k] = q[k];
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < C; k++) vbd_finish(x[k], v[k], dx[k], im[k], h, pp.velocity_decay);
-    }
-#pragma unroll
-    for (int k = 0; k < C; k++) {
-        if (sdf.grid && (fl[k] & F_VALID) && !(fl[k] & F_ROOT)) vbd_sdf(x[k], v[k], sdf, sp);
-        bad |= !finite3(x[k]) || !finite3(v[k]) || !finite4(q[k]);
-    }
-    }  // steps
-
-#pragma unroll
-    for (int k = 0; k < C; k++) {
-        const int64_t g = base + 32LL * k;
-        st.xm[g] = make_float4(x[k].x, x[k].y, x[k].z, im[k]);
-        st.vel[g] = make_float4(v[k].x, v[k].y, v[k].z, 0.f);
-        st.vlast[g] = make_float4(vl[k].x, vl[k].y, vl[k].z, 0.f);
-        st.q[g] = q[k];
-    }
-    if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(st.status, STATUS_NONFINITE);
-}
-
-template <int C>
-__global__ void __launch_bounds__(256) recorded_step_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                            TapeView tp, const StepParams* __restrict__ steps, int nsteps) {
-    recorded_step_body<C, false>(st, pp, sp, sdf, tp, steps, nsteps);
-}
-// The same over groups of tiles: one CTA of K warps per group.
-template <int C>
-__global__ void __launch_bounds__(256) recorded_group_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                             TapeView tp) {
-    recorded_step_body<C, true>(st, pp, sp, sdf, tp, nullptr, 1);
-}
-// The same without a tape: the plain step of few groups (launch_scalar_group).
-template <int C>
-__global__ void __launch_bounds__(256) scalar_group_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                           const StepParams* __restrict__ steps, int nsteps) {
-    recorded_step_body<C, true, false>(st, pp, sp, sdf, TapeView{}, steps, nsteps);
-}
 
 __device__ __forceinline__ float4 zero4() { return make_float4(0.f, 0.f, 0.f, 0.f); }
 __device__ __forceinline__ float3 zero3() { return f3(0.f, 0.f, 0.f); }
@@ -872,18 +567,6 @@ __global__ void __launch_bounds__(NT, MINB) adjoint_step_kernel(DeviceState st, 
 }
 
 // ------------------------------------------------------------------------------------------
-cudaError_t launch_scalar_group(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
-                                int C, int group, cudaStream_t s, const StepParams* d_steps, int nsteps) {
-    if (group < 1 || group > 8 || st.num_tiles % group != 0 || (C != 2 && C != 4)) return cudaErrorInvalidValue;
-    const unsigned blocks = (unsigned)(st.num_tiles / group);
-    if (blocks == 0) return cudaSuccess;
-    if (C == 2)
-        scalar_group_kernel<2><<<blocks, 32 * group, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);
-    else
-        scalar_group_kernel<4><<<blocks, 32 * group, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_fused_record(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
                                 const TapeView& tp, int C, int warps_per_block, cudaStream_t s, int group) {
     if (group > 1) {  // one CTA of `group` warps per group of tiles (the window is whole groups)
@@ -892,9 +575,9 @@ cudaError_t launch_fused_record(const DeviceState& st, const PhysParams& pp, con
         if (tiles == 0) return cudaSuccess;
         const unsigned gblocks = (unsigned)(tiles / group);
         if (C == 2)
-            recorded_group_kernel<2><<<gblocks, 32 * group, 0, s>>>(st, pp, sp, sdf, tp);
+            recorded_step_kernel<2, true><<<gblocks, 32 * group, 0, s>>>(st, pp, sp, sdf, tp);
         else if (C == 4)
-            recorded_group_kernel<4><<<gblocks, 32 * group, 0, s>>>(st, pp, sp, sdf, tp);
+            recorded_step_kernel<4, true><<<gblocks, 32 * group, 0, s>>>(st, pp, sp, sdf, tp);
         else
             return cudaErrorInvalidValue;
         return cudaGetLastError();
@@ -904,9 +587,9 @@ cudaError_t launch_fused_record(const DeviceState& st, const PhysParams& pp, con
     const unsigned blocks = (unsigned)((tiles + warps_per_block - 1) / warps_per_block);
     if (blocks == 0) return cudaSuccess;
     if (C == 2)
-        recorded_step_kernel<2><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, tp, nullptr, 1);
+        recorded_step_kernel<2, false><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, tp);
     else if (C == 4)
-        recorded_step_kernel<4><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, tp, nullptr, 1);
+        recorded_step_kernel<4, false><<<blocks, threads, 0, s>>>(st, pp, sp, sdf, tp);
     else
         return cudaErrorInvalidValue;
     return cudaGetLastError();

@@ -60,9 +60,11 @@ __device__ __forceinline__ float4 qmul_conj_fma(float4 l, float4 r) {
 // trajectories have always had, so a groom moves to the same bits: an FP32 velocity is dx / h, and another
 // rounding of the iterations comes back in it 1e-5 to 1e-4 large on short strands over a few substeps.
 // That order differs between a tile of 2 and of 4 slots a lane, and in the host frame (FROM_E, Y_FIRST,
-// WZ_FIRST and the force in fused_step_body).  Groups of tiles (SHORT) take shorter sums and sqrt.approx: 10.3
-// ms instead of 11.1 for 6,000 strands of 100-300 vertices, 42 substeps of 32 iterations (10.9 before);
-// against 64 bits their positions and orientations err as before (2.7e-7 and 1.6e-6 relative).
+// WZ_FIRST and the force in fused_step_body).  Groups of tiles (SHORT) take shorter sums and sqrt.approx, in
+// every kernel that steps them, a host frame and a recorded step among them: 10.3 ms instead of 10.7 for 6,000
+// strands of 100-300 vertices, 42 substeps of 32 iterations, paired (10.9 with the longer sums in scalar
+// instructions, 10.2 with these); against 64 bits their positions and orientations err as with the longer sums
+// (2.7e-7 and 1.6e-6 relative).  The scalar form of the step (vbd_scalar.cuh) takes the same sums, slot by slot.
 struct V3 {
     float x;
     float2 yz;
@@ -131,19 +133,44 @@ __device__ __forceinline__ Q4 qmul_conj(Q4 l, Q4 r) {
 
 // Half the material axis, d3 / 2 = q e_x q* / 2 (d3_of, vbd_common.cuh); the position update's
 // coefficient carries the other factor of two.
+// SHORT: of a unit quaternion.  It is taken only after an update, which leaves one (a segment that has a next
+// vertex is always updated); the axis of an orientation set from outside is the full one.
 template <bool X_FIRST, bool WZ_FIRST, bool SHORT = false>
 __device__ __forceinline__ V3 half_axis(Q4 q) {
-    if (SHORT) {  // of a unit quaternion: (1/2 - y^2 - z^2, x y + w z, x z - w y)
+    if (SHORT) {  // (1/2 - y^2 - z^2, x y + w z, x z - w y)
         const float2 t = mul2(both(q.xw.x), q.yz);
         return {fmaf(-q.yz.y, q.yz.y, fmaf(-q.yz.x, q.yz.x, 0.5f)),
                 make_float2(fmaf(q.xw.y, q.yz.y, t.x), fmaf(-q.xw.y, q.yz.x, t.y))};
     }
-
     const float x = q.xw.x, y = q.yz.x, z = q.yz.y, w = q.xw.y;
     const float xw = X_FIRST ? fmaf(x, x, __fmul_rn(w, w)) : fmaf(w, w, __fmul_rn(x, x));
     const float d = 0.5f * fmaf(-z, z, fmaf(-y, y, xw));
     if (WZ_FIRST) return {d, make_float2(fmaf(w, z, __fmul_rn(x, y)), fmaf(x, z, __fmul_rn(-w, y)))};
     return {d, fma2(both(x), q.yz, make_float2(__fmul_rn(w, z), __fmul_rn(-w, y)))};
+}
+
+// A vertex's folded coefficients for one substep (see the file comment); zeros for a vertex that does not
+// move.  CHAINED: the order of the force's sum, which differs between the slots of a lane.
+struct VertexFold {
+    float3 F0;
+    float as_, isA, isD;
+};
+template <bool CHAINED>
+__device__ __forceinline__ VertexFold fold_vertex(float im, float h, float damp, float accel, float ddN, float ddP,
+                                                  float3 y, float3 e, float3 eP) {
+    const float a = im != 0.f ? 1.f / (im * h * h) : 0.f;
+    const float sk = __fmul_rn(ddN + ddP, 1.f + damp);
+    VertexFold b;
+    b.as_ = a + sk;
+    b.isA = im != 0.f ? accel / sk : 0.f;
+    b.isD = im != 0.f ? accel / fmaf(3.f, a, sk) - b.isA : 0.f;
+    auto force = [&](float ya, float en, float ep) {
+        const float n = __fmul_rn(ddN, en);  // a segment's product enters both its vertices
+        return CHAINED ? fmaf(-ddP, ep, fmaf(a, ya, n))
+                       : __fsub_rn(__fadd_rn(__fmul_rn(a, ya), n), __fmul_rn(ddP, ep));
+    };
+    b.F0 = f3(force(y.x, e.x, eP.x), force(y.y, e.y, eP.y), force(y.z, e.z, eP.z));
+    return b;
 }
 
 // One position update with folded coefficients (see the file comment).  k2N / k2P are twice kkN / kkP
@@ -234,6 +261,39 @@ struct GroupExchange {
     float4 up[8][XU_N];
     float4 down[8][XD_N];
 };
+
+// A host frame's strands of tile t between the host buffers and the warp's staging area: positions, then
+// velocities, 3 floats per tile position p = lane * C + k (coalesced 4-byte accesses over PCIe).
+template <int C>
+__device__ __forceinline__ void frame_in(const HostIO& hio, int64_t t, float* stage) {
+    const int lane = threadIdx.x & 31;
+    const int r_end = hio.x_in ? hio.run_begin[t + 1] : 0;
+    for (int r = hio.run_begin[t]; r < r_end; r++) {
+        const int4 run = hio.runs[r];
+        const float* gx = hio.x_in + 3LL * run.y;
+        const float* gv = hio.v_in + 3LL * run.y;
+        for (int j = lane; j < 3 * run.z; j += 32) {
+            stage[3 * run.x + j] = gx[j];
+            stage[96 * C + 3 * run.x + j] = gv[j];
+        }
+    }
+    __syncwarp();
+}
+template <int C>
+__device__ __forceinline__ void frame_out(const HostIO& hio, int64_t t, const float* stage) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    const int r_end = hio.run_begin[t + 1];
+    for (int r = hio.run_begin[t]; r < r_end; r++) {
+        const int4 run = hio.runs[r];
+        float* gx = hio.x_out + 3LL * run.y;
+        float* gv = hio.v_out + 3LL * run.y;
+        for (int j = lane; j < 3 * run.z; j += 32) {
+            gx[j] = stage[3 * run.x + j];
+            gv[j] = stage[96 * C + 3 * run.x + j];
+        }
+    }
+}
 
 // Floats of shared memory a slot takes in a fused kernel: position, velocity, last velocity, inverse
 // mass.  A host frame stages the tile's positions and velocities in the same cells before and after.
@@ -419,17 +479,13 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
                 dx[k] = v3(dx0);
                 const float ddP = k > 0 ? ddN[k > 0 ? k - 1 : 0] : ddH;
                 const float3 eP = k > 0 ? e[k > 0 ? k - 1 : 0] : e0;
-                const float a = im != 0.f ? 1.f / (im * h * h) : 0.f;
-                const float sk = __fmul_rn(ddN[k] + ddP, 1.f + damp);
-                as_[k] = a + sk;
-                isA[k] = im != 0.f ? accel / sk : 0.f;
-                isD[k] = im != 0.f ? accel / fmaf(3.f, a, sk) - isA[k] : 0.f;
-                auto force = [&](float ya, float en, float ep) {
-                    const float n = __fmul_rn(ddN[k], en);  // a segment's product enters both its vertices
-                    return SHORT || k == 0 || (C == 2 && !HOSTIO) ? fmaf(-ddP, ep, fmaf(a, ya, n))
-                                            : __fsub_rn(__fadd_rn(__fmul_rn(a, ya), n), __fmul_rn(ddP, ep));
-                };
-                F0[k] = v3(f3(force(y.x, e[k].x, eP.x), force(y.y, e[k].y, eP.y), force(y.z, e[k].z, eP.z)));
+                const VertexFold b = SHORT || k == 0 || (C == 2 && !HOSTIO)
+                                         ? fold_vertex<true>(im, h, damp, accel, ddN[k], ddP, y, e[k], eP)
+                                         : fold_vertex<false>(im, h, damp, accel, ddN[k], ddP, y, e[k], eP);
+                as_[k] = b.as_;
+                isA[k] = b.isA;
+                isD[k] = b.isD;
+                F0[k] = v3(b.F0);
                 const float3 ve = -k2N[k] * e[k];
                 Ve[k] = v3(C == 2 && k == 0 && FROM_E ? f3(e[k].x, e[k].y, FROM_E == 3 ? e[k].z : ve.z) : ve);
                 hd[k] = half_axis<true, false>(q[k]);
@@ -442,15 +498,16 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
         };
         auto orientation = [&](Q4& n, V3& hn, int k, V3 dN, Q4 qP, Q4 qN) {
             const int kp = k > 0 ? k - 1 : 0;
+            constexpr bool Y_FIRST = !JACOBI;  // of the odd slots of 4
             if (C == 2 && k == 0)
-                fused_orientation<SHORT, FROM_E, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qrH, qN, qr[k], use_next_q(k),
-                                               use_prev(k));
+                fused_orientation<SHORT, FROM_E, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qrH, qN,
+                                                                qr[k], use_next_q(k), use_prev(k));
             else if (C == 4 && (k & 1))
-                fused_orientation<SHORT, 0, !JACOBI, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qr[kp], qN, qr[k],
-                                               use_next_q(k), use_prev(k));
+                fused_orientation<SHORT, 0, Y_FIRST, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qr[kp], qN,
+                                                             qr[k], use_next_q(k), use_prev(k));
             else
-                fused_orientation<SHORT, 0, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, k ? qr[kp] : qrH, qN, qr[k],
-                                                use_next_q(k), use_prev(k));
+                fused_orientation<SHORT, 0, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP,
+                                                           k ? qr[kp] : qrH, qN, qr[k], use_next_q(k), use_prev(k));
         };
         Q4 qP = shfl(q[C - 1], from_prev);
         V3 hP = shfl(hd[C - 1], from_prev);  // the previous lane's half axis
@@ -581,17 +638,7 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
             sv[o + 1] = v[k].y;
             sv[o + 2] = v[k].z;
         }
-        __syncwarp();
-        const int r_end = hio.run_begin[tile + 1];
-        for (int r = hio.run_begin[tile]; r < r_end; r++) {
-            const int4 run = hio.runs[r];
-            float* gx = hio.x_out + 3LL * run.y;
-            float* gv = hio.v_out + 3LL * run.y;
-            for (int j = lane; j < 3 * run.z; j += 32) {
-                gx[j] = sx[3 * run.x + j];
-                gv[j] = sv[3 * run.x + j];
-            }
-        }
+        frame_out<C>(hio, tile, sx);
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0) atomicOr(st.status, STATUS_NONFINITE);
 }
@@ -616,17 +663,7 @@ __device__ __forceinline__ void fused_frame(DeviceState st, PhysParams pp, StepP
     const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + w;
     if (t >= st.num_tiles) return;  // uniform per warp (per CTA for groups)
     float* const stage = kami_park + w * (PARK_FLOATS * 32 * C);
-    const int r_end = hio.x_in ? hio.run_begin[t + 1] : 0;
-    for (int r = hio.run_begin[t]; r < r_end; r++) {
-        const int4 run = hio.runs[r];
-        const float* gx = hio.x_in + 3LL * run.y;
-        const float* gv = hio.v_in + 3LL * run.y;
-        for (int j = lane; j < 3 * run.z; j += 32) {
-            stage[3 * run.x + j] = gx[j];
-            stage[3 * 32 * C + 3 * run.x + j] = gv[j];
-        }
-    }
-    __syncwarp();
+    frame_in<C>(hio, t, stage);
     fused_step_body<C, JACOBI, true, GROUPED>(st, pp, sp, sdf, nullptr, 1, hio, t);
 }
 template <int C, bool JACOBI>
@@ -639,7 +676,7 @@ __global__ void __maxnreg__(120) fused_frame_kernel_r120(DeviceState st, PhysPar
                                                         HostIO hio) {
     fused_frame<C, JACOBI>(st, pp, sp, sdf, hio);
 }
-// The same over groups of tiles: one CTA of K warps per group.
+// The same over groups of tiles (4 slots a lane: scalar_frame_group_kernel): one CTA of K warps per group.
 template <int C, bool JACOBI>
 __global__ void __launch_bounds__(256) fused_frame_group_kernel(DeviceState st, PhysParams pp, StepParams sp,
                                                                 SdfParams sdf, HostIO hio) {

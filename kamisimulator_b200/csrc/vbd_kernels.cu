@@ -17,7 +17,7 @@
 #include <mutex>
 #include <tuple>
 
-#include "vbd_fused.cuh"
+#include "vbd_scalar.cuh"
 #include "vbd_kernels.h"
 #include "vbd_math.cuh"
 
@@ -730,44 +730,6 @@ cudaError_t launch_strain_limit(float4* xm, const float4* prm, const int64_t* ro
 
 bool fused_supported(int C) { return C == 2 || C == 4; }
 
-namespace {
-// Launches a frame kernel: one warp per tile.
-template <typename K>
-cudaError_t launch_frame(K kernel, int C, const DeviceState& st, const PhysParams& pp, const StepParams& sp,
-                         const SdfParams& sdf, const HostIO& hio, int warps_per_block, cudaStream_t s) {
-    kernel<<<blocks_for(st.num_tiles, warps_per_block), 32 * warps_per_block, park_bytes(C, warps_per_block), s>>>(
-        st, pp, sp, sdf, hio);
-    return cudaGetLastError();
-}
-}  // namespace
-
-cudaError_t launch_fused_frame(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
-                               const HostIO& hio, int C, bool jacobi, int warps_per_block, cudaStream_t s, int reg_cap,
-                               int group) {
-    if (group > 1) {  // one CTA of `group` warps per group of tiles
-        if (group > 8 || st.num_tiles % group != 0) return cudaErrorInvalidValue;
-        if (st.num_tiles == 0) return cudaSuccess;
-        if (C == 2)
-            return jacobi ? launch_frame(fused_frame_group_kernel<2, true>, 2, st, pp, sp, sdf, hio, group, s)
-                          : launch_frame(fused_frame_group_kernel<2, false>, 2, st, pp, sp, sdf, hio, group, s);
-        if (C == 4)
-            return jacobi ? launch_frame(fused_frame_group_kernel<4, true>, 4, st, pp, sp, sdf, hio, group, s)
-                          : launch_frame(fused_frame_group_kernel<4, false>, 4, st, pp, sp, sdf, hio, group, s);
-        return cudaErrorInvalidValue;
-    }
-    if (blocks_for(st.num_tiles, warps_per_block) == 0) return cudaSuccess;
-    if (reg_cap == 120 && C == 2)
-        return jacobi ? launch_frame(fused_frame_kernel_r120<2, true>, 2, st, pp, sp, sdf, hio, warps_per_block, s)
-                      : launch_frame(fused_frame_kernel_r120<2, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s);
-    if (C == 2)
-        return jacobi ? launch_frame(fused_frame_kernel<2, true>, 2, st, pp, sp, sdf, hio, warps_per_block, s)
-                      : launch_frame(fused_frame_kernel<2, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s);
-    if (C == 4)
-        return jacobi ? launch_frame(fused_frame_kernel<4, true>, 4, st, pp, sp, sdf, hio, warps_per_block, s)
-                      : launch_frame(fused_frame_kernel<4, false>, 4, st, pp, sp, sdf, hio, warps_per_block, s);
-    return cudaErrorInvalidValue;
-}
-
 // Resident CTAs of `kernel` at `threads` threads on the current device (cached per device, kernel
 // and block size), times the SM count.
 static cudaError_t resident_ctas(const void* kernel, int threads, size_t smem, int64_t* out) {
@@ -799,6 +761,75 @@ static cudaError_t persistent_grid(const void* kernel, int threads, size_t smem,
     if (e != cudaSuccess) return e;
     *grid = (unsigned)std::min<int64_t>(units, resident);
     return cudaSuccess;
+}
+
+// Whether the plain step of `groups` groups runs in scalar instructions (the results are the same to the bit).
+// Scalar and paired, 42 substeps of 32 iterations at 4 slots a lane, colour2, us by groups of 4 tiles: 24 732 and
+// 868, 169 1220 and 1267, 322 1896 and 2019, 794 3612 and 3712, 2,400 10,203 and 10,360: the group's barriers make
+// the chain of dependent instructions the bound, and the paired instructions' moves between layouts make it
+// longer.  Paired where the groups are a little more than one resident wave: the scalar kernel's CTAs of an SM
+// end together, so a second wave of up to one CTA an SM is scheduled two to an SM and takes as long as the first
+// (365 groups 2387 and 2042, 402 groups 2414 and 2050).  Jacobi, with two barriers an iteration instead of three,
+// and the register caps stay paired.
+static cudaError_t scalar_groups(unsigned groups, int threads, int C, bool jacobi, int reg_cap, bool* scalar) {
+    *scalar = false;
+    if (C != 4 || jacobi || reg_cap > 1) return cudaSuccess;
+    int dev = 0, sms = 0;
+    int64_t resident = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = resident_ctas((const void*)scalar_group_kernel<4>, threads, 0, &resident);
+    *scalar = groups <= resident + sms / 4 || groups > resident + sms;
+    return e;
+}
+
+namespace {
+// Launches a frame kernel: one warp per tile.
+template <typename K>
+cudaError_t launch_frame(K kernel, int C, const DeviceState& st, const PhysParams& pp, const StepParams& sp,
+                         const SdfParams& sdf, const HostIO& hio, int warps_per_block, cudaStream_t s) {
+    kernel<<<blocks_for(st.num_tiles, warps_per_block), 32 * warps_per_block, park_bytes(C, warps_per_block), s>>>(
+        st, pp, sp, sdf, hio);
+    return cudaGetLastError();
+}
+// The scalar frame kernel of groups of tiles.
+template <typename K>
+cudaError_t launch_group_frame(K kernel, int C, const DeviceState& st, const PhysParams& pp, const StepParams& sp,
+                               const SdfParams& sdf, const HostIO& hio, int group, cudaStream_t s) {
+    const size_t smem = sizeof(float) * 6 * 32 * (size_t)C * group;
+    unsigned grid = 0;
+    cudaError_t e = persistent_grid((const void*)kernel, 32 * group, smem, st.num_tiles / group, &grid);
+    if (e != cudaSuccess) return e;
+    kernel<<<grid, 32 * group, smem, s>>>(st, pp, sp, sdf, hio);
+    return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_fused_frame(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
+                               const HostIO& hio, int C, bool jacobi, int warps_per_block, cudaStream_t s, int reg_cap,
+                               int group) {
+    if (group > 1) {  // one CTA of `group` warps per group of tiles
+        if (group > 8 || st.num_tiles % group != 0) return cudaErrorInvalidValue;
+        if (st.num_tiles == 0) return cudaSuccess;
+        if (C == 2)
+            return jacobi ? launch_frame(fused_frame_group_kernel<2, true>, 2, st, pp, sp, sdf, hio, group, s)
+                          : launch_frame(fused_frame_group_kernel<2, false>, 2, st, pp, sp, sdf, hio, group, s);
+        if (C == 4)
+            return jacobi ? launch_group_frame(scalar_frame_group_kernel<4, true>, 4, st, pp, sp, sdf, hio, group, s)
+                          : launch_group_frame(scalar_frame_group_kernel<4, false>, 4, st, pp, sp, sdf, hio, group, s);
+        return cudaErrorInvalidValue;
+    }
+    if (blocks_for(st.num_tiles, warps_per_block) == 0) return cudaSuccess;
+    if (reg_cap == 120 && C == 2)
+        return jacobi ? launch_frame(fused_frame_kernel_r120<2, true>, 2, st, pp, sp, sdf, hio, warps_per_block, s)
+                      : launch_frame(fused_frame_kernel_r120<2, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s);
+    if (C == 2)
+        return jacobi ? launch_frame(fused_frame_kernel<2, true>, 2, st, pp, sp, sdf, hio, warps_per_block, s)
+                      : launch_frame(fused_frame_kernel<2, false>, 2, st, pp, sp, sdf, hio, warps_per_block, s);
+    if (C == 4)
+        return jacobi ? launch_frame(fused_frame_kernel<4, true>, 4, st, pp, sp, sdf, hio, warps_per_block, s)
+                      : launch_frame(fused_frame_kernel<4, false>, 4, st, pp, sp, sdf, hio, warps_per_block, s);
+    return cudaErrorInvalidValue;
 }
 
 template <typename K>
@@ -850,15 +881,13 @@ cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const
         const unsigned gblocks = (unsigned)(st.num_tiles / group);
         if (gblocks == 0) return cudaSuccess;
         const int gthreads = 32 * group;
-        // Up to one warp a scheduler (4 an SM) a group's time is its chain of dependent instructions, and the
-        // paired ones, with the moves between their layouts, make the colour2 chain longer: 42 substeps of 32
-        // iterations take 815 us in scalar FP32 and 873 paired at 480 tiles.  With more tiles the schedulers
-        // share issue slots: 1317 against 1258 us at 652 tiles, 10.9 ms against 10.35 at 9,600.  Jacobi: paired
-        // at every size (828 against 767 us at 480 tiles).
-        int dev = 0, sms = 0;
-        if (!jacobi && reg_cap <= 1 && cudaGetDevice(&dev) == cudaSuccess &&
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && st.num_tiles <= 4LL * sms)
-            return launch_scalar_group(st, pp, sp, sdf, C, group, s, d_steps, nsteps);
+        bool scalar = false;
+        cudaError_t e = scalar_groups(gblocks, gthreads, C, jacobi, reg_cap, &scalar);
+        if (e != cudaSuccess) return e;
+        if (scalar) {
+            scalar_group_kernel<4><<<gblocks, gthreads, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);
+            return cudaGetLastError();
+        }
 #define KAMI_GROUP_LAUNCH(KERNEL, CC)                                                                   \
     do {                                                                                                \
         if (jacobi)                                                                                     \

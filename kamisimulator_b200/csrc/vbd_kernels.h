@@ -60,9 +60,6 @@ cudaError_t launch_fused_frame(const DeviceState& st, const PhysParams& pp, cons
                                const HostIO& hio, int C, bool jacobi, int warps_per_block, cudaStream_t s, int reg_cap,
                                int group = 1);
 
-// The colour2 step of groups of tiles in scalar FP32 (vbd_adjoint.cu): the same calls as launch_fused_step's groups.
-cudaError_t launch_scalar_group(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
-                                int C, int group, cudaStream_t s, const StepParams* d_steps, int nsteps);
 // group > 1: groups of tiles, one CTA of `group` warps each (2, 4 or 8);
 // the tape window must be whole groups.
 cudaError_t launch_fused_record(const DeviceState& st, const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,

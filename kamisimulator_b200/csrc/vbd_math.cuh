@@ -11,18 +11,19 @@ namespace kami {
 // the reference keeps it in d_vels).  Pinned vertices keep dx = h v and y = v.
 __device__ __forceinline__ void vbd_predict(float3 x, float3 v, float3 vlast, float inv_mass, const PhysParams& pp,
                                             float h, float last_h, float time, float3& dx, float3& y) {
+    // (sums of products are written with fmaf: every kernel that predicts rounds alike)
     float windx = 0.f;
     if (pp.wind_peak != 0.f) {
         // the reference evaluates the cosines in double (2 * M_PI promotes), iteration.cu:22-25
-        float wy = x.y > 0.f ? (float)cos(2.0 * 3.14159265358979323846 * (double)(pp.wind_yf * x.y + pp.wind_tf * time)) : 0.f;
-        float wz = (float)cos(2.0 * 3.14159265358979323846 * (double)(pp.wind_zf * fabsf(x.z) + pp.wind_tf * time));
+        const float phase = __fmul_rn(pp.wind_tf, time);
+        float wy = x.y > 0.f ? (float)cos(2.0 * 3.14159265358979323846 * (double)fmaf(pp.wind_yf, x.y, phase)) : 0.f;
+        float wz = (float)cos(2.0 * 3.14159265358979323846 * (double)fmaf(pp.wind_zf, fabsf(x.z), phase));
         float prod = wy * wz;
         float sg = prod > 0.f ? 1.f : (prod < 0.f ? -1.f : 0.f);
         float pw = powf(prod, pp.wind_sharp) * sg;
-        windx = pp.wind_peak * ((0.f < pw) ? pw : 0.f);
+        windx = __fmul_rn(pp.wind_peak, (0.f < pw) ? pw : 0.f);
     }
-    float3 ext = f3(pp.gx + windx, pp.gy, pp.gz) * pp.ext_mult;
-    // (written with fmaf: every kernel that predicts rounds alike)
+    float3 ext = f3(__fadd_rn(pp.gx, windx), pp.gy, pp.gz) * pp.ext_mult;
     dx = f3(__fmul_rn(h, v.x), __fmul_rn(h, v.y), __fmul_rn(h, v.z));
     y = v;
     if (inv_mass != 0.f) {

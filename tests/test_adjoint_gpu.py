@@ -522,3 +522,53 @@ def test_stiffness_fit_reduces_loss_on_the_2000_strand_workload():
         losses.append(loss.item())
     assert losses[-1] < 0.8 * losses[0], losses
     solver.close()
+
+
+@pytest.mark.parametrize("slots", [2, 4])
+def test_recorded_step_equals_the_plain_step(slots):
+    """A recorded step is the plain step, bit for bit, on tiles of 64 and of 128 slots: the checkpoints
+    of a rollout and its recomputed segments are the same numbers."""
+    g = helpers.soft_groom(61, (3, 60), seed=slots)
+    st = helpers.soft_settings(num_itr=5, max_h=1 / 120, sdf=synth.sphere_sdf(48, threshold=2e-3),
+                               wind=(2.0, 1.0, 0.7, 0.4, 3.0), slots_per_lane=slots)
+    s = helpers.gpu_solver(g, st, form="fused", velocities=helpers.random_velocities(g, 0.2, seed=2))
+    try:
+        start = s.get_state()
+        for _ in range(2):
+            s.step(1 / 60)
+        plain = s.get_state()
+        s.set_state(start)
+        s.tape_reserve(4, 0)
+        for _ in range(2):
+            s.step_record(1 / 60)
+        recorded = s.get_state()
+    finally:
+        s.close()
+    assert np.isfinite(plain[:-4]).all() and not np.array_equal(plain, start)
+    np.testing.assert_array_equal(recorded, plain)
+
+
+@pytest.mark.parametrize("mode", ["budget_0", "windows"])
+def test_first_and_second_rollout_on_long_strands_are_the_same(mode):
+    """A rollout that records nothing in its forward pass gives the same positions and gradient on a fresh handle
+    as on one that already has a tape, on more groups of tiles than one wave of CTAs holds."""
+    import torch
+
+    from kamisimulator_b200.autograd import rollout_positions
+
+    g, st, solver, unit, strand_of, init, v0 = _setup(num_strands=700, lengths=(150, 250), seed=29, num_itr=4)
+    c = torch.tensor(np.random.default_rng(4).normal(size=(g.num_vertices, 3)), dtype=torch.float32, device="cuda")
+    scale0 = np.random.default_rng(3).uniform(0.7, 1.4, g.num_strands).astype(np.float32)
+    kw = dict(tape_budget_bytes=0) if mode == "budget_0" else dict(tiles_per_chunk=solver.tile_count() // 2)
+    out = []
+    try:
+        for _ in range(2):
+            scale = torch.tensor(scale0, device="cuda", requires_grad=True)
+            x = rollout_positions(scale, solver, unit, strand_of, init, 3, 1 / 60, checkpoint_every=2, **kw)
+            (c * x).sum().backward()
+            out.append((x.detach().cpu().numpy(), solver.get_rest_darboux_grad()))
+    finally:
+        solver.close()
+    assert np.isfinite(out[0][1]).all()
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])

@@ -169,3 +169,50 @@ def test_few_and_many_groups_match_the_oracle(strands):
     s = helpers.soft_settings(num_itr=4, max_h=1 / 120, sdf=synth.sphere_sdf(32, radius=0.09, half_extent=0.6))
     ex, et = _lockstep(g, s, "fused", 1, 1 / 60)
     assert ex <= 1e-5 and et <= 1e-5, (ex, et)
+
+
+def _same_steps(g, st, tuning, schedule, dt):
+    """The state after two steps by every call that steps a handle, from the same start."""
+    import torch
+
+    v = helpers.random_velocities(g, 0.1, seed=3)
+    out = {}
+    calls = ("step", "step_n", "persistent", "frame", "pageable") + (("taped", "record") if schedule == "colour2" else ())
+    for call in calls:
+        s = helpers.gpu_solver(g, dict(st, schedule=schedule), form="fused", velocities=v)
+        try:
+            s.set_tuning(*tuning)
+            if call == "persistent":
+                s.set_launch_mode(1)
+            if call in ("taped", "record"):
+                s.tape_reserve(4, 0)
+            if call == "step_n":
+                s.step_n(dt, 2)
+            elif call in ("frame", "pageable"):
+                x, vv = s.get_positions_velocities()
+                if call == "frame":
+                    x, vv = torch.from_numpy(x.copy()).pin_memory(), torch.from_numpy(vv.copy()).pin_memory()
+                for _ in range(2):
+                    s.step_host(dt, x, vv)
+            else:
+                for _ in range(2):
+                    s.step_record(dt) if call == "record" else s.step(dt)
+            out[call] = s.get_state()
+        finally:
+            s.close()
+    return out
+
+
+@pytest.mark.parametrize("schedule", ["colour2", "jacobi"])
+@pytest.mark.parametrize("tuning", [(4, 1, 2, 1), (4, 1, 2, 168), (2, 1, 2, 1)])
+@pytest.mark.parametrize("strands", [3, 660, 900])
+def test_every_call_steps_long_strands_alike(strands, tuning, schedule):
+    """One, two and more waves of groups (the sizes between which the kernel of a plain step changes): a step,
+    several steps of one launch, resident CTAs, a host frame from page-locked and from pageable arrays, a step on
+    a handle with a tape and a recorded step give the same state, bit for bit, with wind, body and substeps."""
+    g = synth.groom_strands(np.random.default_rng(9), np.random.default_rng(strands).integers(150, 251, strands))
+    st = _settings(num_itr=4, max_h=1 / 240, wind=(2.0, 1.0, 0.7, 0.4, 3.0), sdf=synth.sphere_sdf(64, threshold=2e-3))
+    out = _same_steps(g, st, tuning, schedule, 1 / 120)
+    assert np.isfinite(out["step"][:-4]).all()
+    for call, state in out.items():
+        np.testing.assert_array_equal(state, out["step"], err_msg=call)
