@@ -191,6 +191,9 @@ __device__ __forceinline__ void scalar_step_body(DeviceState st, PhysParams pp, 
         ddH = dk.x;
         k2H = dk.y;
     }
+    const bool hp0 = fl[0] & F_HAS_PREV;  // (a shuffle gives lane 0 its own values)
+    ddH = hp0 ? ddH : 0.f;
+    k2H = hp0 ? k2H : 0.f;
 
     const float accel = pp.accel_ratio;
     bool bad = false;
@@ -219,6 +222,7 @@ __device__ __forceinline__ void scalar_step_body(DeviceState st, PhysParams pp, 
                 group_sync();
                 eH = xyz(up_get(XU_E, f4(eH)));
             }
+            eH = hp0 ? eH : f3(0.f, 0.f, 0.f);
 #pragma unroll
             for (int k = 0; k < C; k++) {
                 float3 y;

@@ -524,13 +524,14 @@ def test_stiffness_fit_reduces_loss_on_the_2000_strand_workload():
     solver.close()
 
 
+@pytest.mark.parametrize("pin_roots", [True, False])
 @pytest.mark.parametrize("slots", [2, 4])
-def test_recorded_step_equals_the_plain_step(slots):
-    """A recorded step is the plain step, bit for bit, on tiles of 64 and of 128 slots: the checkpoints
-    of a rollout and its recomputed segments are the same numbers."""
+def test_recorded_step_equals_the_plain_step(slots, pin_roots):
+    """A recorded step is the plain step, bit for bit, on tiles of 64 and of 128 slots, whether the strands' roots
+    move or not: the checkpoints of a rollout and its recomputed segments are the same numbers."""
     g = helpers.soft_groom(61, (3, 60), seed=slots)
     st = helpers.soft_settings(num_itr=5, max_h=1 / 120, sdf=synth.sphere_sdf(48, threshold=2e-3),
-                               wind=(2.0, 1.0, 0.7, 0.4, 3.0), slots_per_lane=slots)
+                               wind=(2.0, 1.0, 0.7, 0.4, 3.0), pin_roots=pin_roots, slots_per_lane=slots)
     s = helpers.gpu_solver(g, st, form="fused", velocities=helpers.random_velocities(g, 0.2, seed=2))
     try:
         start = s.get_state()

@@ -216,3 +216,31 @@ def test_every_call_steps_long_strands_alike(strands, tuning, schedule):
     assert np.isfinite(out["step"][:-4]).all()
     for call, state in out.items():
         np.testing.assert_array_equal(state, out["step"], err_msg=call)
+
+
+@pytest.mark.parametrize("slots", [2, 4])
+@pytest.mark.parametrize("strands", [3, 400])
+def test_unpinned_long_strands_match_the_oracle(strands, slots):
+    """Strand roots that move, lane 0 of a group's first tile among them: a vertex without a previous segment takes
+    no force from one.  The bar is that of one step; the recorded step equals it."""
+    g = helpers.soft_groom(strands, (150, 250), seed=strands)
+    st = helpers.soft_settings(num_itr=4, max_h=1 / 120, pin_roots=False)
+    v = helpers.random_velocities(g, 0.1, seed=2)
+    o = helpers.oracle_sim(g, st, np.float32, v)
+    s = helpers.gpu_solver(g, st, form="fused", velocities=v)
+    try:
+        s.set_tuning(slots_per_lane=slots)
+        start = s.get_state()
+        o.advance(1 / 60)
+        s.step(1 / 60)
+        x, _ = s.get_positions_velocities()
+        q, plain = s.get_orientations(), s.get_state()
+        s.set_state(start)
+        s.tape_reserve(2, 0)
+        s.step_record(1 / 60)
+        recorded = s.get_state()
+    finally:
+        s.close()
+    assert np.abs(x - o.x).max() <= helpers.POS_TOL
+    assert np.abs(twist_angles(o.q, q)).max() <= helpers.TWIST_TOL
+    np.testing.assert_array_equal(recorded, plain)
