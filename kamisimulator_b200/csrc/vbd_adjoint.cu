@@ -293,6 +293,7 @@ __global__ void __launch_bounds__(NT, MINB) adjoint_step_kernel(DeviceState st, 
         qrH = up_get(AU_QR, qrH, qrH);
         ddH = up_get(AU_DD, make_float4(ddH, 0.f, 0.f, 0.f), make_float4(ddH, 0.f, 0.f, 0.f)).x;
     }
+    ddH = (fl[0] & F_HAS_PREV) ? ddH : 0.f;  // (a shuffle gives lane 0 its own values)
     const float h = sp.h;
     const float damp = pp.damping / h;
     const float accel = pp.accel_ratio;

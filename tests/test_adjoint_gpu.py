@@ -573,3 +573,36 @@ def test_first_and_second_rollout_on_long_strands_are_the_same(mode):
     assert np.isfinite(out[0][1]).all()
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("num_strands,lengths,group", [(24, (6, 20), 1), (6, (150, 250), 2)])
+def test_unpinned_roots_gradient_matches_fp64_autograd(monkeypatch, num_strands, lengths, group):
+    """Roots that move, lane 0 of a tile among them: the adjoint of a vertex without a previous segment takes
+    nothing from one.  The restatement run in FP32 is 3e-6 from FP64 here, so the bar is the gradient's own."""
+    import torch
+
+    from kamisimulator_b200.autograd import rollout_positions
+    from oracle import oracle as orc
+
+    g = helpers.soft_groom(num_strands, lengths, seed=5 if group == 1 else 23, young_scale=1e-3)
+    st = dict(num_itr=5, max_h=1 / 60, gravity=(0.3, -0.4, -9.81), radius=40e-6, sdf=None)
+    v0 = helpers.random_velocities(g, 0.15, seed=6 if group == 1 else 24)
+    solver = helpers.gpu_solver(g, dict(st, pin_roots=False), form="fused", velocities=v0)
+    assert solver.tiles_per_group() == group
+    rng = np.random.default_rng(0)
+    scale0 = rng.uniform(0.7, 1.4, num_strands).astype(np.float32)
+    c = rng.normal(size=(g.num_vertices, 3))
+    try:
+        unit = torch.tensor(solver.get_rest_darboux(), device="cuda")
+        strand_of = torch.tensor(np.repeat(np.arange(num_strands), np.diff(g.strand_begin)), device="cuda")
+        init = torch.tensor(solver.get_state(), device="cuda")
+        scale = torch.tensor(scale0, device="cuda", requires_grad=True)
+        x = rollout_positions(scale, solver, unit, strand_of, init, 4, 1 / 60, checkpoint_every=2)
+        (torch.tensor(c, dtype=torch.float32, device="cuda") * x).sum().backward()
+    finally:
+        solver.close()
+    configure = orc.configure
+    monkeypatch.setattr(orc, "configure", lambda *a, **k: configure(*a, **dict(k, pin_roots=False)))
+    _, g_ref, *_ = _torch_reference(g, st, v0, scale0, 4, c)
+    g_gpu = scale.grad.cpu().numpy()
+    assert _rel(g_gpu, g_ref) <= GRAD_TOL, (_rel(g_gpu, g_ref), g_gpu[:5], g_ref[:5])
