@@ -199,12 +199,15 @@ __device__ __forceinline__ void fused_position(V3& dx, V3 F0, float ddN, float k
 // One orientation update (quaternionLambdaItr).  qrP and qr are zero where the previous / next segment
 // is missing, so its product vanishes.  With the signs s1, s2 of the two products (cosserat.cu:316-335),
 // b = s1 P1 + s2 P2 = s1 (P1 + s1 s2 P2), and s1 is applied to the normalised result, which is linear
-// in b.  A sign test reads the sign bit of the negated dot product (set where the product is positive;
-// x - x gives +0, which counts as not positive).  R = V b e_x + lambda b with V = (V, 0), written out.
+// in b.  A dot product of zero (an exact half turn between two segments) counts as not positive.  The signs are
+// compared in predicates (colour2: 93.6 us for 10,000 x 64, 95.8 with sign bits) or, where that leaves too few
+// registers for the whole lane at once (Jacobi: 275 us for 5,000 x 200, 308 with predicates), in sign bits.
+// R = V b e_x + lambda b with V = (V, 0), written out.
 // FROM_E: the components of Ve (all 3, or x and y) that hold the segment vector e instead of m2k e.
 template <bool SHORT, int FROM_E, bool Y_FIRST, bool WZ_FIRST>
 __device__ __forceinline__ void fused_orientation(Q4& q, V3& h, bool upd, V3 Ve, float m2k, V3 dx, V3 dxN, Q4 qPrev,
                                                   Q4 qrP, Q4 qNext, Q4 qr, bool use_n, bool use_p) {
+    constexpr bool SIGN_BITS = WZ_FIRST;  // Jacobi
     const V3 d = {dxN.x - dx.x, sub2(dxN.yz, dx.yz)};
     V3 V;
     if (FROM_E == 3)
@@ -219,8 +222,10 @@ __device__ __forceinline__ void fused_orientation(Q4& q, V3& h, bool upd, V3 Ve,
     if (!use_p) P1 = zero;
     if (!use_n) P2 = zero;
     const float2 t1 = fma2(q.yz, P1.yz, mul2(q.xw, P1.xw)), t2 = fma2(q.yz, P2.yz, mul2(q.xw, P2.xw));
-    const uint32_t g1 = __float_as_uint(-t1.x - t1.y), g2 = __float_as_uint(-t2.x - t2.y);
-    const float s12 = __uint_as_float(((g1 ^ g2) & 0x80000000u) | 0x3f800000u);
+    const float dot1 = t1.x + t1.y, dot2 = t2.x + t2.y;
+    const bool pos1 = dot1 > 0.f, pos2 = dot2 > 0.f;
+    const uint32_t g1 = __float_as_uint(0.f - dot1), g2 = __float_as_uint(0.f - dot2);  // sign bit: positive
+    const float s12 = SIGN_BITS ? __uint_as_float(((g1 ^ g2) & 0x80000000u) | 0x3f800000u) : pos1 == pos2 ? 1.f : -1.f;
     const Q4 b = {fma2(both(s12), P2.yz, P1.yz), fma2(both(s12), P2.xw, P1.xw)};
     const float vv = norm2<Y_FIRST>(V), bb = SHORT ? short_norm2(b) : norm2(b);
     const float lambda = SHORT ? sqrt_ftz(vv) + sqrt_ftz(bb)
@@ -242,7 +247,7 @@ __device__ __forceinline__ void fused_orientation(Q4& q, V3& h, bool upd, V3 Ve,
         R = {fma2(both(lambda), b.yz, Pzy), fma2(both(lambda), b.xw, Pwx)};
     }
     const float inv = rsqrt_ftz(SHORT ? short_norm2(R) : norm2(R));
-    const float2 si = both(__uint_as_float(__float_as_uint(inv) ^ (~g1 & 0x80000000u)));
+    const float2 si = both(SIGN_BITS ? __uint_as_float(__float_as_uint(inv) ^ (~g1 & 0x80000000u)) : pos1 ? inv : -inv);
     if (upd) {
         q.yz = mul2(si, R.yz);
         q.xw = mul2(si, R.xw);

@@ -349,3 +349,30 @@ def test_device_boundary_arrays_equal_the_host_ones(skew, strands, length):
         np.testing.assert_array_equal(s.get_state().view(np.int32), state.view(np.int32))
     finally:
         s.close()
+
+
+@pytest.mark.parametrize("slots,schedule", [(2, "colour2"), (4, "colour2"), (2, "jacobi"), (4, "jacobi")])
+@pytest.mark.parametrize("length", [7, 150])
+def test_exact_half_turns_count_as_not_positive(length, slots, schedule):
+    """Straight rods whose segments are turned against their neighbours by exactly half a turn about their axis:
+    the dot products of the sign tests are zeros of either sign, and only a positive one gives +1
+    (cosserat.cu:316-335).  The sign decides that of the new orientation, so it is compared with the oracle's
+    sign and all; one iteration rounds a unit quaternion a few times (1e-6)."""
+    g = synth.cantilever(5, length)
+    st = dict(num_itr=1, max_h=1 / 120, gravity=(0.0, 0.0, -9.81), radius=40e-6, schedule=schedule)
+    o = helpers.oracle_sim(g, st, np.float32)
+    q = np.zeros((g.num_vertices, 4), np.float32)
+    q[0::2, 3], q[1::2, 0] = 1.0, 1.0
+    state = o.state()
+    np.testing.assert_allclose(state["q"], np.tile([0.0, 0.0, 0.0, 1.0], (g.num_vertices, 1)), atol=1e-7)
+    o.load_state(dict(state, q=q))
+    o.advance(1 / 120)
+    s = helpers.gpu_solver(g, st, form="fused")
+    try:
+        s.set_tuning(slots_per_lane=slots)
+        s.set_orientations(q)
+        s.step(1 / 120)
+        got = s.get_orientations()
+    finally:
+        s.close()
+    np.testing.assert_allclose(got, o.q, rtol=0, atol=1e-6)
