@@ -15,6 +15,10 @@ LIB_PATH = os.path.join(_HERE, "_ref", "libkami_ref.so")
 _lib = None
 
 
+class NotBuilt(RuntimeError):
+    """The library is not there: it is built from the reference's sources (oracle/ref/Makefile)."""
+
+
 def available():
     return os.path.exists(LIB_PATH)
 
@@ -22,10 +26,8 @@ def available():
 def load():
     global _lib
     if _lib is None:
-        if not available():  # as the tests that ask available() first
-            import pytest
-
-            pytest.skip("oracle/_ref not built (needs the reference sources)")
+        if not available():
+            raise NotBuilt("oracle/_ref not built (needs the reference sources)")
         lib = ctypes.CDLL(LIB_PATH)
         vp, i32, i64, f32 = ctypes.c_void_p, ctypes.c_int32, ctypes.c_int64, ctypes.c_float
         lib.ref_create.restype = vp

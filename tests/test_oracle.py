@@ -353,3 +353,13 @@ def test_strain_limiting_restatement_on_a_hand_case():
     assert abs(d6 - 0.5) < 1e-6  # |(1, 0.6, 0.5) - (1, 0, 1)| = 0.781 > 1.1 x 0.5: pulled to 0.5
     # a tolerance that covers every strain changes nothing
     np.testing.assert_array_equal(orc.strain_limit(x, sb, l0, 10.0), x)
+
+
+def test_a_missing_reference_library_is_an_error_not_a_skip(monkeypatch):
+    """The loader raises; only the test run turns that into a skip, with its reason (tests/conftest.py)."""
+    from oracle import ref_sim
+
+    monkeypatch.setattr(ref_sim, "_lib", None)
+    monkeypatch.setattr(ref_sim, "LIB_PATH", ref_sim.LIB_PATH + ".missing")
+    with pytest.raises(ref_sim.NotBuilt, match="not built"):
+        ref_sim.strain_limit(np.zeros((3, 3), np.float32), [0, 3], np.ones(3, np.float32))

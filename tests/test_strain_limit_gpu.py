@@ -167,3 +167,39 @@ def test_strain_limit_on_a_batch_handle_matches_each_groom_on_its_own():
             s.close()
     assert np.abs(want - np.concatenate([x0, x1])).max() > 1e-4
     np.testing.assert_array_equal(xb, want)
+
+
+@pytest.mark.parametrize("layout", ["c2", "c4", "sweep", "groups"])
+def test_strain_limit_matches_the_oracle_on_every_layout(layout):
+    """Stretched strands against the oracle alone (no reference library needed), strands across groups of
+    tiles among them: a vertex's two roundings of 0.4 m (1.5e-8 each) add up over 200 vertices like a random
+    walk, well inside the bar."""
+    g = synth.groom(64, 200, seed=3) if layout == "groups" else helpers.soft_groom(300, (6, 64), seed=21)
+    x = _strained(g, 8, 1.0, 1.3)
+    form, tuning = {"c2": ("fused", (2, 4, 1, 1)), "c4": ("fused", (4, 4, 1, 1)), "sweep": ("sweep", None),
+                    "groups": ("fused", (2, 1, 1, 1))}[layout]
+    ours = _gpu_strain_limit(g, x, 0.1, form, tuning)
+    want = orc.strain_limit(x, g.strand_begin, _rest_lengths(g), 0.1)
+    assert (np.abs(want - x).max(axis=1) > 0).mean() > 0.5
+    assert np.abs(ours - want).max() <= ORACLE_TOL
+
+
+def test_strain_limit_sees_the_positions_of_the_step_before_it():
+    """A step and the limit queued behind it equal the limit on a handle that was given the step's positions."""
+    g = helpers.soft_groom(120, (8, 40), seed=9)
+    st = helpers.soft_settings(sdf=synth.sphere_sdf(64, threshold=2e-3))
+    a, b = helpers.gpu_solver(g, st), helpers.gpu_solver(g, st)
+    try:
+        for _ in range(3):
+            a.step(1 / 60)
+            b.step(1 / 60)
+            x, v = b.get_positions_velocities()
+            a.strain_limit(0.01)
+            got = a.get_positions_velocities()[0]
+            b.set_positions_velocities(x, v)
+            b.strain_limit(0.01)
+            np.testing.assert_array_equal(got, b.get_positions_velocities()[0])
+            assert np.abs(got - x).max() > 0
+    finally:
+        a.close()
+        b.close()
