@@ -1632,7 +1632,9 @@ kami_status kami_vbd_get_tiles_per_group(kami_vbd_handle h, int32_t* tiles_per_g
 // The tape window's slots [s0, s0 + n) and the slot -> vertex map for the scatters and gathers of
 // kami_vbd_backward and kami_vbd_restore_tape_window; *vert_of stays null when the window covers the
 // whole groom.
-static kami_status slot_vertices(kami_vbd_solver* h) {  // builds d_vert_of for the current layout
+static kami_status window_slots(kami_vbd_solver* h, const int64_t** vert_of, int64_t* s0, int64_t* n) {
+    *vert_of = nullptr;
+    if (h->win_begin == 0 && h->win_end >= h->layout.num_tiles) return KAMI_OK;
     if (!h->d_vert_of || h->vert_of_C != h->layout.C || h->vert_of_K != h->layout.K) {
         if (h->d_vert_of) cudaFree(h->d_vert_of);
         h->d_vert_of = nullptr;
@@ -1641,12 +1643,6 @@ static kami_status slot_vertices(kami_vbd_solver* h) {  // builds d_vert_of for 
         h->vert_of_C = h->layout.C;
         h->vert_of_K = h->layout.K;
     }
-    return KAMI_OK;
-}
-static kami_status window_slots(kami_vbd_solver* h, const int64_t** vert_of, int64_t* s0, int64_t* n) {
-    *vert_of = nullptr;
-    if (h->win_begin == 0 && h->win_end >= h->layout.num_tiles) return KAMI_OK;
-    KAMI_TRY(slot_vertices(h));
     const int64_t T = 32LL * h->layout.C;
     *vert_of = h->d_vert_of;
     *s0 = h->win_begin * T;
@@ -1735,8 +1731,7 @@ kami_status kami_vbd_backward(kami_vbd_handle h, float* adj_x, float* adj_v, flo
         BoundaryArrays a;
         for (int k = 0; k < 3; k++) a.add(adj3[k], ins3[k], 3);
         a.add(h->d_gq, adj_q, 4);
-        KAMI_TRY(slot_vertices(h));
-        KAMI_CUDA(launch_fill_arrays(a, h->d_vert_of, (int64_t)S, h->stream), "scatter adjoint");
+        KAMI_CUDA(launch_fill_arrays(a, h->d_slot_of, h->nv, h->d_prm, (int64_t)S, h->stream), "scatter adjoint");
     } else {
         for (int a = 0; a < 3; a++) {
             KAMI_CUDA(cudaMemsetAsync(adj3[a], 0, sizeof(float4) * S, h->stream), "adjoint reset");

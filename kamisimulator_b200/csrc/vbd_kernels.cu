@@ -538,17 +538,19 @@ __global__ void scatter_arrays_kernel(BoundaryArrays a, const int64_t* __restric
         a.slots[k][g] = make_float4(f[0], f[1], f[2], a.comps[k] == 4 ? f[3] : a.slots[k][g].w);
     }
 }
-// The same into every slot, zero in padding slots (the adjoint's buffers); vert_of as below.
-__global__ void fill_arrays_kernel(BoundaryArrays a, const int64_t* __restrict__ vert_of, int64_t num_slots) {
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= num_slots) return;
-    const int64_t i = vert_of[g];
+// The same into every slot: zero in padding slots, which their flags tell (the adjoint's buffers).
+__global__ void fill_arrays_kernel(BoundaryArrays a, const int64_t* __restrict__ slot_of, int64_t nv,
+                                   const float4* __restrict__ prm, int64_t num_slots) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool padding = i < num_slots && !(__float_as_uint(prm[i].w) & F_VALID);
+    const int64_t g = i < nv ? slot_of[i] : -1;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         if (k >= a.n) break;
+        if (padding) a.slots[k][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (g < 0) continue;
         const float* f = a.flat[k] + a.comps[k] * i;
-        a.slots[k][g] = i < 0 ? make_float4(0.f, 0.f, 0.f, 0.f)
-                              : make_float4(f[0], f[1], f[2], a.comps[k] == 4 ? f[3] : 0.f);
+        a.slots[k][g] = make_float4(f[0], f[1], f[2], a.comps[k] == 4 ? f[3] : 0.f);
     }
 }
 // Tape windows: the slots [s0, s0 + n) of a window and the boundary vertices they hold (vert_of: the
@@ -1009,9 +1011,10 @@ cudaError_t launch_scatter_arrays(const BoundaryArrays& a, const int64_t* slot_o
     scatter_arrays_kernel<<<blocks_for(nv, 256), 256, 0, s>>>(a, slot_of, nv);
     return cudaGetLastError();
 }
-cudaError_t launch_fill_arrays(const BoundaryArrays& a, const int64_t* vert_of, int64_t num_slots, cudaStream_t s) {
+cudaError_t launch_fill_arrays(const BoundaryArrays& a, const int64_t* slot_of, int64_t nv, const float4* prm,
+                               int64_t num_slots, cudaStream_t s) {
     if (num_slots == 0) return cudaSuccess;
-    fill_arrays_kernel<<<blocks_for(num_slots, 256), 256, 0, s>>>(a, vert_of, num_slots);
+    fill_arrays_kernel<<<blocks_for(num_slots, 256), 256, 0, s>>>(a, slot_of, nv, prm, num_slots);
     return cudaGetLastError();
 }
 cudaError_t launch_vert_of(const int64_t* slot_of, int64_t* vert_of, int64_t nv, int64_t num_slots, cudaStream_t s) {

@@ -113,7 +113,7 @@ cudaError_t launch_gather4(const float4* src, float4* dst, const int64_t* slot_o
 
 // Up to four arrays between device arrays of the caller (flat: comps floats per boundary vertex, 3 or 4)
 // and the tile slots.  gather: also *status to status_out and the clock to clock_out (each may be null).
-// scatter: a 3-component array keeps the slot's .w.  fill: every slot, zero where vert_of is -1.
+// scatter: a 3-component array keeps the slot's .w.  fill: every slot (num_slots >= nv), zero in padding.
 struct BoundaryArrays {
     float4* slots[4];
     float* flat[4];
@@ -128,7 +128,8 @@ struct BoundaryArrays {
 cudaError_t launch_gather_arrays(const BoundaryArrays& a, const int64_t* slot_of, int64_t nv, const int* status,
                                  int* status_out, float4 clock, float* clock_out, cudaStream_t s);
 cudaError_t launch_scatter_arrays(const BoundaryArrays& a, const int64_t* slot_of, int64_t nv, cudaStream_t s);
-cudaError_t launch_fill_arrays(const BoundaryArrays& a, const int64_t* vert_of, int64_t num_slots, cudaStream_t s);
+cudaError_t launch_fill_arrays(const BoundaryArrays& a, const int64_t* slot_of, int64_t nv, const float4* prm,
+                               int64_t num_slots, cudaStream_t s);
 
 // Tape windows: vert_of (num_slots entries) = the boundary vertex of every slot, -1 for padding; and
 // slots [s0, s0 + n) <-> their vertices in a caller's boundary array of `comps` (3 or 4) floats per

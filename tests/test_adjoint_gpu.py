@@ -606,3 +606,25 @@ def test_unpinned_roots_gradient_matches_fp64_autograd(monkeypatch, num_strands,
     _, g_ref, *_ = _torch_reference(g, st, v0, scale0, 4, c)
     g_gpu = scale.grad.cpu().numpy()
     assert _rel(g_gpu, g_ref) <= GRAD_TOL, (_rel(g_gpu, g_ref), g_gpu[:5], g_ref[:5])
+
+
+def test_first_backward_of_a_whole_groom_allocates_nothing():
+    """The adjoint arrays of a whole groom go to the tile slots and back through the handle's own vertex map: a
+    first kami_vbd_backward takes no device memory for the handle's life (a slot map would be 4 MB here)."""
+    import torch
+
+    for strands in (8, 8000):  # the first, small one loads the kernels
+        s = helpers.gpu_solver(synth.groom(strands, 64, seed=2), dict(num_itr=2, max_h=1 / 120), form="fused")
+        try:
+            s.tape_reserve(1, 0)
+            s.step_record(1 / 120)
+            adj = [torch.ones((s.num_vertices, n), device="cuda") for n in (3, 3, 3, 4)]
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info()[0]
+            s.backward(*adj)
+            torch.cuda.synchronize()
+            taken = free - torch.cuda.mem_get_info()[0]
+            assert all(torch.isfinite(a).all() for a in adj)
+        finally:
+            s.close()
+    assert taken == 0
