@@ -95,3 +95,36 @@ def test_gpu_bake_skips_no_nearest_triangle(kind, dims, pad):
     phi, _ = orc.sdf_bake(V, T, dims, g.grid_min, g.grid_max)
     big = max(np.abs(lo).max(), np.abs(hi).max())
     assert np.abs(np.abs(g.phi) - np.abs(phi)).max() <= 2e-6 + 1e-6 * big
+
+
+def _scan_of_all(V, T, dims, lo, hi):
+    """The bakes with nothing skipped: meshes of 16 consecutive triangles, which are one cluster each and tested
+    whole."""
+    for c in range(0, len(T), 16):
+        used, local = np.unique(T[c:c + 16], return_inverse=True)
+        yield vbd.bake_sdf(V[used], local.reshape(-1, 3).astype(np.int32), dims, lo, hi)
+
+
+@pytest.mark.parametrize("kind,dims,pad", [
+    ("tetrahedron", (5, 3, 7), 0.05), ("sphere", (15, 14, 13), 0.02), ("sphere", (8, 8, 4), 3.0),
+    ("slivers", (13, 11, 10), 0.05), ("away", (10, 9, 5), 0.05), ("rough", (17, 12, 14), 0.0), ("tiny", (9, 9, 9), 2e-8)])
+def test_gpu_bake_equals_a_scan_over_all_triangles(kind, dims, pad):
+    """Skipping clusters changes no bit: the magnitude at every node, and the gradient where a node lies inside the
+    mesh (there it points to the nearest triangle, so a wrong one shows; a patch of 16 triangles has no inside of
+    its own, but its pseudonormals give the mesh's sign almost everywhere).  The sign is that
+    of the FP64 distance, where that is clear of the coordinates' rounding (a few 6e-8 of the largest one)."""
+    V, T = _mesh_of(kind) if kind != "tiny" else synth.icosphere(3, 1e-7)
+    lo, hi = V.min(0) - np.float32(pad), V.max(0) + np.float32(pad)
+    g = vbd.bake_sdf(V, T, dims, lo, hi)
+    parts = list(_scan_of_all(V, T, dims, lo, hi))
+    nearest = np.min([np.abs(p.phi) for p in parts], axis=0)
+    np.testing.assert_array_equal(np.abs(g.phi).view(np.int32), nearest.view(np.int32))
+    at = [(np.abs(p.phi) == nearest) & (p.phi < 0) for p in parts]  # (squares that differ may have one root)
+    inside, shown = g.phi < 0, (g.phi < 0) & np.any(at, axis=0)
+    if kind in ("sphere", "rough", "tiny") and pad < 1:
+        assert shown.sum() >= 0.9 * inside.sum() > 50
+    same = np.any([a & (p.grad == g.grad).all(-1) for a, p in zip(at, parts)], axis=0)
+    assert same[shown].all()
+    exact, _ = orc.sdf_bake(V, T, dims, g.grid_min, g.grid_max)
+    clear = np.abs(exact) > 1e-6 * max(np.abs(lo).max(), np.abs(hi).max())
+    np.testing.assert_array_equal(np.sign(g.phi[clear]), np.sign(exact[clear]))
