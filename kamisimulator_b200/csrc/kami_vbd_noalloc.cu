@@ -107,7 +107,7 @@ __global__ void noalloc_predict_kernel(NoAllocArgs a, PhysParams pp, StepParams 
     if (i >= a.nv) return;
     float3 x = ld3(a.x, i), v = ld3(a.v, i), vl = ld3(a.vl, i);
     float3 dx, y;
-    vbd_predict(x, v, vl, a.im[i], pp, sp.h, sp.last_h, sp.time, dx, y);
+    vbd_predict<false>(x, v, vl, a.im[i], pp, sp.h, sp.last_h, sp.time, dx, y);
     st3(a.vl, i, v);
     a.scratch[i] = make_float4(y.x, y.y, y.z, 0.f);
     a.scratch[kMaxV + i] = make_float4(dx.x, dx.y, dx.z, 0.f);

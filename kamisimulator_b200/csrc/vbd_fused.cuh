@@ -479,7 +479,7 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
                 float3 dx0, y;
                 const float3 v = parked3(PARK_V, k);
                 const float im = cell(PARK_IM, k);
-                vbd_predict(x[k], v, parked3(PARK_VL, k), im, pp, h, sp.last_h, sp.time, dx0, y);
+                vbd_predict<C == 4>(x[k], v, parked3(PARK_VL, k), im, pp, h, sp.last_h, sp.time, dx0, y);
                 park3(PARK_VL, k, v);
                 dx[k] = v3(dx0);
                 const float ddP = k > 0 ? ddN[k > 0 ? k - 1 : 0] : ddH;

@@ -39,7 +39,7 @@ __global__ void sweep_predict_kernel(DeviceState st, float4* y4, float4* dx4, co
     float3 v = xyz(st.vel[g]);
     float3 vl = xyz(st.vlast[g]);
     float3 dx, y;
-    vbd_predict(xyz(xm), v, vl, xm.w, pp, sp.h, sp.last_h, sp.time, dx, y);
+    vbd_predict<false>(xyz(xm), v, vl, xm.w, pp, sp.h, sp.last_h, sp.time, dx, y);
     st.vlast[g] = make_float4(v.x, v.y, v.z, 0.f);
     y4[g] = make_float4(y.x, y.y, y.z, 0.f);
     dx4[g] = make_float4(dx.x, dx.y, dx.z, 0.f);

@@ -8,16 +8,20 @@ namespace kami {
 
 // Inertial predict + initial guess of one vertex: initItr, YarnBall/sim/iteration.cu:8-59.
 // Returns dx (initial guess of the displacement) and y (= y - x, the inertial target displacement;
-// the reference keeps it in d_vels).  Pinned vertices keep dx = h v and y = v.
+// the reference keeps it in d_vels).  Pinned vertices keep dx = h v and y = v.  Sums of products are written with
+// fmaf, so that every kernel rounds them alike; PHASE_FIRST: the order of the wind's, which has always differed
+// between tiles of 2 and of 4 slots a lane.
+template <bool PHASE_FIRST>
 __device__ __forceinline__ void vbd_predict(float3 x, float3 v, float3 vlast, float inv_mass, const PhysParams& pp,
                                             float h, float last_h, float time, float3& dx, float3& y) {
-    // (sums of products are written with fmaf: every kernel that predicts rounds alike)
     float windx = 0.f;
     if (pp.wind_peak != 0.f) {
         // the reference evaluates the cosines in double (2 * M_PI promotes), iteration.cu:22-25
-        const float phase = __fmul_rn(pp.wind_tf, time);
-        float wy = x.y > 0.f ? (float)cos(2.0 * 3.14159265358979323846 * (double)fmaf(pp.wind_yf, x.y, phase)) : 0.f;
-        float wz = (float)cos(2.0 * 3.14159265358979323846 * (double)fmaf(pp.wind_zf, fabsf(x.z), phase));
+        auto phase = [&](float f, float p) {
+            return PHASE_FIRST ? fmaf(f, p, __fmul_rn(pp.wind_tf, time)) : fmaf(pp.wind_tf, time, __fmul_rn(f, p));
+        };
+        float wy = x.y > 0.f ? (float)cos(2.0 * 3.14159265358979323846 * (double)phase(pp.wind_yf, x.y)) : 0.f;
+        float wz = (float)cos(2.0 * 3.14159265358979323846 * (double)phase(pp.wind_zf, fabsf(x.z)));
         float prod = wy * wz;
         float sg = prod > 0.f ? 1.f : (prod < 0.f ? -1.f : 0.f);
         float pw = powf(prod, pp.wind_sharp) * sg;

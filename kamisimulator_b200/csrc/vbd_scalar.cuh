@@ -226,7 +226,7 @@ __device__ __forceinline__ void scalar_step_body(DeviceState st, PhysParams pp, 
 #pragma unroll
             for (int k = 0; k < C; k++) {
                 float3 y;
-                vbd_predict(x[k], v[k], vl[k], im[k], pp, h, sp.last_h, sp.time, dx[k], y);
+                vbd_predict<C == 4>(x[k], v[k], vl[k], im[k], pp, h, sp.last_h, sp.time, dx[k], y);
                 vl[k] = v[k];
                 const float ddP = k > 0 ? ddN[k > 0 ? k - 1 : 0] : ddH;
                 const float3 eP = k > 0 ? e[k > 0 ? k - 1 : 0] : eH;
