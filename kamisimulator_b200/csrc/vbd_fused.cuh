@@ -199,15 +199,16 @@ __device__ __forceinline__ void fused_position(V3& dx, V3 F0, float ddN, float k
 // One orientation update (quaternionLambdaItr).  qrP and qr are zero where the previous / next segment
 // is missing, so its product vanishes.  With the signs s1, s2 of the two products (cosserat.cu:316-335),
 // b = s1 P1 + s2 P2 = s1 (P1 + s1 s2 P2), and s1 is applied to the normalised result, which is linear
-// in b.  A dot product of zero (an exact half turn between two segments) counts as not positive.  The signs are
-// compared in predicates (colour2: 93.6 us for 10,000 x 64, 95.8 with sign bits) or, where that leaves too few
-// registers for the whole lane at once (Jacobi: 275 us for 5,000 x 200, 308 with predicates), in sign bits.
-// R = V b e_x + lambda b with V = (V, 0), written out.
+// in b.  R = V b e_x + lambda b with V = (V, 0), written out.  A dot product of zero (an exact half turn between
+// two segments) counts as not positive.  Each sign is a predicate or the sign bit of 0 - dot, whichever leaves
+// the shorter step; both bits, s1 s2 as bits and s1 as a predicate, both predicates: 10,000 x 64 (2 slots a
+// lane) 94.8, 93.0 and 93.1 us, 2,000 uneven strands in 3 substeps 47.0, 45.4 and 46.7; 3,000 x 96 (4 slots)
+// 81.7, 82.4 and 80.3; Jacobi, groups, 5,000 x 200 274 with bits and 308 with predicates.
 // FROM_E: the components of Ve (all 3, or x and y) that hold the segment vector e instead of m2k e.
-template <bool SHORT, int FROM_E, bool Y_FIRST, bool WZ_FIRST>
+template <bool SHORT, int FROM_E, bool Y_FIRST, bool WZ_FIRST, bool S12_BITS>
 __device__ __forceinline__ void fused_orientation(Q4& q, V3& h, bool upd, V3 Ve, float m2k, V3 dx, V3 dxN, Q4 qPrev,
                                                   Q4 qrP, Q4 qNext, Q4 qr, bool use_n, bool use_p) {
-    constexpr bool SIGN_BITS = WZ_FIRST;  // Jacobi
+    constexpr bool S1_BITS = WZ_FIRST;  // Jacobi
     const V3 d = {dxN.x - dx.x, sub2(dxN.yz, dx.yz)};
     V3 V;
     if (FROM_E == 3)
@@ -225,7 +226,7 @@ __device__ __forceinline__ void fused_orientation(Q4& q, V3& h, bool upd, V3 Ve,
     const float dot1 = t1.x + t1.y, dot2 = t2.x + t2.y;
     const bool pos1 = dot1 > 0.f, pos2 = dot2 > 0.f;
     const uint32_t g1 = __float_as_uint(0.f - dot1), g2 = __float_as_uint(0.f - dot2);  // sign bit: positive
-    const float s12 = SIGN_BITS ? __uint_as_float(((g1 ^ g2) & 0x80000000u) | 0x3f800000u) : pos1 == pos2 ? 1.f : -1.f;
+    const float s12 = S12_BITS ? __uint_as_float(((g1 ^ g2) & 0x80000000u) | 0x3f800000u) : pos1 == pos2 ? 1.f : -1.f;
     const Q4 b = {fma2(both(s12), P2.yz, P1.yz), fma2(both(s12), P2.xw, P1.xw)};
     const float vv = norm2<Y_FIRST>(V), bb = SHORT ? short_norm2(b) : norm2(b);
     const float lambda = SHORT ? sqrt_ftz(vv) + sqrt_ftz(bb)
@@ -247,7 +248,7 @@ __device__ __forceinline__ void fused_orientation(Q4& q, V3& h, bool upd, V3 Ve,
         R = {fma2(both(lambda), b.yz, Pzy), fma2(both(lambda), b.xw, Pwx)};
     }
     const float inv = rsqrt_ftz(SHORT ? short_norm2(R) : norm2(R));
-    const float2 si = both(SIGN_BITS ? __uint_as_float(__float_as_uint(inv) ^ (~g1 & 0x80000000u)) : pos1 ? inv : -inv);
+    const float2 si = both(S1_BITS ? __uint_as_float(__float_as_uint(inv) ^ (~g1 & 0x80000000u)) : pos1 ? inv : -inv);
     if (upd) {
         q.yz = mul2(si, R.yz);
         q.xw = mul2(si, R.xw);
@@ -504,15 +505,17 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
         auto orientation = [&](Q4& n, V3& hn, int k, V3 dN, Q4 qP, Q4 qN) {
             const int kp = k > 0 ? k - 1 : 0;
             constexpr bool Y_FIRST = !JACOBI;  // of the odd slots of 4
+            constexpr bool BITS = (C == 2 && !SHORT) || JACOBI;
             if (C == 2 && k == 0)
-                fused_orientation<SHORT, FROM_E, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qrH, qN,
-                                                                qr[k], use_next_q(k), use_prev(k));
+                fused_orientation<SHORT, FROM_E, false, JACOBI, BITS>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qrH,
+                                                                      qN, qr[k], use_next_q(k), use_prev(k));
             else if (C == 4 && (k & 1))
-                fused_orientation<SHORT, 0, Y_FIRST, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qr[kp], qN,
-                                                             qr[k], use_next_q(k), use_prev(k));
+                fused_orientation<SHORT, 0, Y_FIRST, JACOBI, BITS>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP, qr[kp],
+                                                                   qN, qr[k], use_next_q(k), use_prev(k));
             else
-                fused_orientation<SHORT, 0, false, JACOBI>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP,
-                                                           k ? qr[kp] : qrH, qN, qr[k], use_next_q(k), use_prev(k));
+                fused_orientation<SHORT, 0, false, JACOBI, BITS>(n, hn, upd(k), Ve[k], -k2N[k], dx[k], dN, qP,
+                                                                 k ? qr[kp] : qrH, qN, qr[k], use_next_q(k),
+                                                                 use_prev(k));
         };
         Q4 qP = shfl(q[C - 1], from_prev);
         V3 hP = shfl(hd[C - 1], from_prev);  // the previous lane's half axis
