@@ -765,24 +765,39 @@ static cudaError_t persistent_grid(const void* kernel, int threads, size_t smem,
     return cudaSuccess;
 }
 
-// Whether the plain step of `groups` groups runs in scalar instructions (the results are the same to the bit).
-// Scalar and paired, 42 substeps of 32 iterations at 4 slots a lane, colour2, us by groups of 4 tiles: 24 732 and
-// 868, 169 1220 and 1267, 322 1896 and 2019, 794 3612 and 3712, 2,400 10,203 and 10,360: the group's barriers make
-// the chain of dependent instructions the bound, and the paired instructions' moves between layouts make it
-// longer.  Paired where the groups are a little more than one resident wave: the scalar kernel's CTAs of an SM
-// end together, so a second wave of up to one CTA an SM is scheduled two to an SM and takes as long as the first
-// (365 groups 2387 and 2042, 402 groups 2414 and 2050).  Jacobi, with two barriers an iteration instead of three,
-// and the register caps stay paired.
-static cudaError_t scalar_groups(unsigned groups, int threads, int C, bool jacobi, int reg_cap, bool* scalar) {
-    *scalar = false;
-    if (C != 4 || jacobi || reg_cap > 1) return cudaSuccess;
+// Whether the groups past the `resident` ones are to be a launch of their own, with `alone` bytes of shared memory
+// so that they come one to an SM.  The resident CTAs of an SM end together, so the hardware puts a second wave
+// several to an SM even where it has one CTA an SM or fewer, and it takes as long as the first.  (Later waves
+// find the SMs out of step.)
+static cudaError_t spread_second_wave(const void* kernel, int threads, size_t smem, int64_t groups, int64_t* resident,
+                                      size_t* alone, bool* spread) {
     int dev = 0, sms = 0;
-    int64_t resident = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = resident_ctas((const void*)scalar_group_kernel<4>, threads, 0, &resident);
-    *scalar = groups <= resident + sms / 4 || groups > resident + sms;
-    return e;
+    if (e == cudaSuccess) e = resident_ctas(kernel, threads, smem, resident);
+    if (e != cudaSuccess) return e;
+    *alone = 116 * 1024;  // more than half of an SM's 227 KB
+    *spread = groups > *resident + sms / 4 && groups <= *resident + sms;
+    return *spread ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*alone) : cudaSuccess;
+}
+
+// The colour2 step of groups of tiles with 4 slots a lane and no register cap, in scalar instructions (the results
+// are the paired kernels' to the bit).  Scalar and paired, 42 substeps of 32 iterations, us by groups of 4 tiles: 24
+// 732 and 868, 169 1220 and 1267, 322 1896 and 2019, 794 3612 and 3712, 2,400 10,203 and 10,360: the group's
+// barriers make the chain of dependent instructions the bound, and the paired instructions' moves between layouts
+// make it longer.  Jacobi, with two barriers an iteration instead of three, and the register caps stay paired.
+static cudaError_t launch_scalar_groups(const DeviceState& st, const PhysParams& pp, const StepParams& sp,
+                                        const SdfParams& sdf, unsigned groups, int threads, cudaStream_t s,
+                                        const StepParams* d_steps, int nsteps) {
+    int64_t resident = 0;
+    size_t alone = 0;
+    bool spread = false;
+    cudaError_t e = spread_second_wave((const void*)scalar_group_kernel<4>, threads, 0, groups, &resident, &alone, &spread);
+    if (e != cudaSuccess) return e;
+    const unsigned first = spread ? (unsigned)resident : groups;
+    scalar_group_kernel<4><<<first, threads, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps, 0);
+    if (spread) scalar_group_kernel<4><<<groups - first, threads, alone, s>>>(st, pp, sp, sdf, d_steps, nsteps, (int)first);
+    return cudaGetLastError();
 }
 
 namespace {
@@ -798,11 +813,16 @@ cudaError_t launch_frame(K kernel, int C, const DeviceState& st, const PhysParam
 template <typename K>
 cudaError_t launch_group_frame(K kernel, int C, const DeviceState& st, const PhysParams& pp, const StepParams& sp,
                                const SdfParams& sdf, const HostIO& hio, int group, cudaStream_t s) {
+    const int threads = 32 * group, groups = (int)(st.num_tiles / group);
     const size_t smem = sizeof(float) * 6 * 32 * (size_t)C * group;
-    unsigned grid = 0;
-    cudaError_t e = persistent_grid((const void*)kernel, 32 * group, smem, st.num_tiles / group, &grid);
+    int64_t resident = 0;
+    size_t alone = 0;
+    bool spread = false;
+    cudaError_t e = spread_second_wave((const void*)kernel, threads, smem, groups, &resident, &alone, &spread);
     if (e != cudaSuccess) return e;
-    kernel<<<grid, 32 * group, smem, s>>>(st, pp, sp, sdf, hio);
+    const int first = spread ? (int)resident : groups;
+    kernel<<<(unsigned)std::min<int64_t>(first, resident), threads, smem, s>>>(st, pp, sp, sdf, hio, 0, first);
+    if (spread) kernel<<<(unsigned)(groups - first), threads, alone, s>>>(st, pp, sp, sdf, hio, first, groups);
     return cudaGetLastError();
 }
 }  // namespace
@@ -859,10 +879,15 @@ static cudaError_t launch_fused_persistent(const DeviceState& st, const PhysPara
                   : launch_persistent(KERNEL<CC, false>, units, threads, park_bytes(CC, W), s, st, pp, sp, sdf, d_steps, nsteps)
     if (group > 1) {
         if (group > 8 || st.num_tiles % group != 0) return cudaErrorInvalidValue;
+        if (C == 4 && !jacobi && reg_cap != 168)  // (launch_scalar_groups)
+            return launch_persistent(scalar_persistent_group_kernel<4>, units, threads, 0, s, st, pp, sp, sdf, d_steps,
+                                     nsteps);
         if (C == 2 && reg_cap == 120) KAMI_PERSIST(fused_persistent_group_kernel_r120, 2);
         if (C == 4 && reg_cap == 168) KAMI_PERSIST(fused_persistent_group_kernel_r168, 4);
         if (C == 2) KAMI_PERSIST(fused_persistent_group_kernel, 2);
-        if (C == 4) KAMI_PERSIST(fused_persistent_group_kernel, 4);
+        if (C == 4)
+            return launch_persistent(fused_persistent_group_kernel<4, true>, units, threads, park_bytes(4, W), s, st, pp,
+                                     sp, sdf, d_steps, nsteps);
         return cudaErrorInvalidValue;
     }
     if (C == 2 && reg_cap == 120) KAMI_PERSIST(fused_persistent_kernel_r120, 2);
@@ -883,19 +908,14 @@ cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const
         const unsigned gblocks = (unsigned)(st.num_tiles / group);
         if (gblocks == 0) return cudaSuccess;
         const int gthreads = 32 * group;
-        bool scalar = false;
-        cudaError_t e = scalar_groups(gblocks, gthreads, C, jacobi, reg_cap, &scalar);
-        if (e != cudaSuccess) return e;
-        if (scalar) {
-            scalar_group_kernel<4><<<gblocks, gthreads, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps);
-            return cudaGetLastError();
-        }
+        if (C == 4 && !jacobi && reg_cap != 168)
+            return launch_scalar_groups(st, pp, sp, sdf, gblocks, gthreads, s, d_steps, nsteps);
 #define KAMI_GROUP_LAUNCH(KERNEL, CC)                                                                   \
     do {                                                                                                \
         if (jacobi)                                                                                     \
-            KERNEL<CC, true><<<gblocks, gthreads, park_bytes(CC, group), s>>>(st, pp, sp, sdf, d_steps, nsteps);             \
+            KERNEL<CC, true><<<gblocks, gthreads, park_bytes(CC, group), s>>>(st, pp, sp, sdf, d_steps, nsteps); \
         else                                                                                            \
-            KERNEL<CC, false><<<gblocks, gthreads, park_bytes(CC, group), s>>>(st, pp, sp, sdf, d_steps, nsteps);            \
+            KERNEL<CC, false><<<gblocks, gthreads, park_bytes(CC, group), s>>>(st, pp, sp, sdf, d_steps, nsteps); \
     } while (0)
         if (C == 2 && reg_cap == 120)
             KAMI_GROUP_LAUNCH(fused_group_kernel_r120, 2);
@@ -904,7 +924,7 @@ cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const
         else if (C == 2)
             KAMI_GROUP_LAUNCH(fused_group_kernel, 2);
         else if (C == 4)
-            KAMI_GROUP_LAUNCH(fused_group_kernel, 4);
+            fused_group_kernel<4, true><<<gblocks, gthreads, park_bytes(4, group), s>>>(st, pp, sp, sdf, d_steps, nsteps);
         else
             return cudaErrorInvalidValue;
 #undef KAMI_GROUP_LAUNCH

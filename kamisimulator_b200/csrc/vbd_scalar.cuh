@@ -6,7 +6,7 @@
 // step, a host frame or several steps of one launch can follow one another in any mix.
 //
 // What it is for.  A group's barriers make the chain of dependent instructions the bound, which the paired form's
-// moves between layouts lengthen (launch_fused_step has the times of both); and a recorded step is bound by the
+// moves between layouts lengthen (launch_scalar_groups has the times of both); and a recorded step is bound by the
 // tape it writes.
 #pragma once
 #include "vbd_fused.cuh"
@@ -396,24 +396,35 @@ __global__ void __launch_bounds__(256) recorded_step_kernel(DeviceState st, Phys
     if (tile >= st.num_tiles) return;  // uniform per warp (per CTA for groups: num_tiles is a multiple of K)
     scalar_step_body<C, false, GROUPED, true, false>(st, pp, sp, sdf, tp, nullptr, 1, HostIO{}, nullptr, tile);
 }
-// The plain step of groups of tiles, one CTA of K warps per group (the grid is whole groups).
+// The plain step of groups of tiles, one CTA of K warps per group, from group `first` on.
 template <int C>
 __global__ void __launch_bounds__(256) scalar_group_kernel(DeviceState st, PhysParams pp, StepParams sp, SdfParams sdf,
-                                                           const StepParams* __restrict__ steps, int nsteps) {
-    const int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+                                                           const StepParams* __restrict__ steps, int nsteps, int first) {
+    const int64_t tile = (int64_t)(first + blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
     scalar_step_body<C, false, true, false, false>(st, pp, sp, sdf, TapeView{}, steps, nsteps, HostIO{}, nullptr, tile);
 }
-// A host frame of groups of tiles: resident CTAs loop over the groups, since a second wave that the hardware
-// schedules comes two CTAs to an SM (the CTAs of an SM end together) and takes as long as the first.  Frames of
-// 42 substeps from and to host arrays, both schedules: 900 strands (365 groups) 2.61 and 2.67 ms scheduled by the
-// hardware, 2.12 and 2.17 looping (2.25 and 2.32 paired); 60 strands 0.78 and 0.78 (0.94 and 0.96 paired).
+// The same with resident CTAs that loop over the groups (LAUNCH_PERSISTENT).
+template <int C>
+__global__ void __launch_bounds__(256) scalar_persistent_group_kernel(DeviceState st, PhysParams pp, StepParams sp,
+                                                                      SdfParams sdf,
+                                                                      const StepParams* __restrict__ steps, int nsteps) {
+    const int K = blockDim.x >> 5;
+    for (int u = blockIdx.x; (int64_t)u * K < st.num_tiles; u += gridDim.x) {
+        scalar_step_body<C, false, true, false, false>(st, pp, sp, sdf, TapeView{}, steps, nsteps, HostIO{}, nullptr,
+                                                       (int64_t)u * K + (threadIdx.x >> 5));
+        __syncthreads();  // the group exchange area is reused by the next group
+    }
+}
+// A host frame of the groups [first, last): resident CTAs loop over them, which keeps the SMs evenly filled.  Frames
+// of 42 substeps from and to host arrays, colour2 and Jacobi: 900 strands (365 groups) 2.61 and 2.67 ms with a CTA
+// for each group, 2.12 and 2.17 looping (2.25 and 2.32 paired); 60 strands 0.78 and 0.78 (0.94 and 0.96 paired).
 template <int C, bool JACOBI>
 __global__ void __launch_bounds__(256) scalar_frame_group_kernel(DeviceState st, PhysParams pp, StepParams sp,
-                                                                 SdfParams sdf, HostIO hio) {
+                                                                 SdfParams sdf, HostIO hio, int first, int last) {
     extern __shared__ float scalar_stage[];
     float* const stage = scalar_stage + (threadIdx.x >> 5) * (6 * 32 * C);
     const int K = blockDim.x >> 5;
-    for (int u = blockIdx.x; (int64_t)u * K < st.num_tiles; u += gridDim.x) {
+    for (int u = first + blockIdx.x; u < last; u += gridDim.x) {
         const int64_t t = (int64_t)u * K + (threadIdx.x >> 5);
         frame_in<C>(hio, t, stage);
         scalar_step_body<C, JACOBI, true, false, true>(st, pp, sp, sdf, TapeView{}, nullptr, 1, hio, stage, t);
