@@ -1379,7 +1379,8 @@ kami_status kami_vbd_set_tuning(kami_vbd_handle h, int32_t slots_per_lane, int32
                         "register_cap must be 0 (unchanged), 1 or 2 (none), 120 or 168");
         if (register_cap == 2 && (h->layout.C != 4 || h->layout.K != 1 || h->schedule != KAMI_SCHEDULE_COLOUR2))
             return fail(KAMI_ERR_UNSUPPORTED,
-                        "register_cap 2 (the packed step) takes colour2 with 4 slots per lane on single tiles");
+                        "register_cap 2 (once a packed variant, the plain kernel now) takes colour2 with 4 slots per lane on "
+                        "single tiles");
         const int cap = register_cap == 1 ? 0 : register_cap;
         if (cap != h->reg_cap) drop_graphs(h);
         h->reg_cap = cap;

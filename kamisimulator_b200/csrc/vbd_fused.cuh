@@ -308,9 +308,9 @@ constexpr size_t park_bytes(int C, int warps) { return sizeof(float) * PARK_FLOA
 enum : uint32_t { F_MOVES = 1u << 31 };  // in the kernels' flags: the vertex has mass
 
 // One launch runs `nsteps` consecutive steps, step j with clock and body transform steps[j] (or
-// `sp` when steps is null), keeping the tile's state on chip between them.  HOSTIO steps tile `frame_tile` of a host frame (fused_frame_kernel):
-// the warp's shared memory holds the tile's positions then velocities from the host buffers of `hio`, 3
-// floats per tile position p = lane * C + k, and the step writes its results back to the host buffers
+// `sp` when steps is null), keeping the tile's state on chip between them.  HOSTIO steps tile `frame_tile` of
+// a host frame (fused_frame_kernel): the warp's shared memory holds the tile's positions then velocities from
+// the host buffers of `hio`, 3 floats per tile position p = lane * C + k, and the step writes its results back to the host buffers
 // through the same area, as well as to the device state.  Every fused kernel is launched with
 // park_bytes(C, warps) of dynamic shared memory.
 // EXPLICIT_TILE steps tile `frame_tile` (the persistent kernels' tile loop) instead of the launch's own.
@@ -550,7 +550,8 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
                     position(dx[k], k, k == C - 1 ? dxN : dx[k + 1 < C ? k + 1 : k], dx[k - 1], hd[k - 1]);
                 // orientations, even segments
 #pragma unroll
-                for (int k = 0; k < C; k += 2) orientation(q[k], hd[k], k, dx[k + 1], k ? q[k > 0 ? k - 1 : 0] : qP, q[k + 1]);
+                for (int k = 0; k < C; k += 2)
+                    orientation(q[k], hd[k], k, dx[k + 1], k ? q[k > 0 ? k - 1 : 0] : qP, q[k + 1]);
                 // orientations, odd segments
                 Q4 qN = shfl(q[0], from_next_q);
                 if (GROUPED) {

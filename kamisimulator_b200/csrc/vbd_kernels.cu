@@ -431,8 +431,8 @@ cudaError_t launch_sweep_iteration(const DeviceState& st, const float4* y4, cons
     const int64_t warps = st.num_tiles * (C / 2);
     chained = chained && (warps <= 6LL * sms || warps >= 24LL * sms);
     if (jacobi)
-        return launch_chained(chained, sweep_iteration_jacobi_kernel, (unsigned)st.num_tiles, T / 2, smem, s, st, y4, q_in,
-                              q_out, dx_in, dx_out, d_sp, pp, C);
+        return launch_chained(chained, sweep_iteration_jacobi_kernel, (unsigned)st.num_tiles, T / 2, smem, s, st, y4,
+                              q_in, q_out, dx_in, dx_out, d_sp, pp, C);
     return launch_chained(chained, sweep_iteration_kernel, (unsigned)st.num_tiles, T / 2, smem, s, st, y4, q_out, dx_in,
                           dx_out, d_sp, pp, C);
 }
@@ -499,9 +499,10 @@ __global__ void gather4_kernel(const float4* __restrict__ src, float4* __restric
 // Several of a call's arrays at once, between the caller's device arrays and the tile slots: one launch,
 // and each vertex's slot is looked up once.  Memory bound: 8 B of index and 28 B an array and vertex
 // (a step of 640,000 vertices and the read of its positions and velocities: 129 us of wall time with two
-// gathers into a staging buffer and two copies out of it, 104 with this, of which 11 are the status word's
-// pageable copy; 64 x 32 vertices 40 and 20).  Boundary arrays are read and written as floats (any 4-byte alignment).  The
-// gather's first thread also hands out what the call reports beside them: the status word and a clock.
+// gathers into a staging buffer, two copies out of it and a pageable copy of the status word, which alone was 11,
+// and 104 with this; 64 x 32 vertices 40 and 20).  Boundary arrays are read and written as floats (any 4-byte
+// alignment).  The gather's first thread also hands out what the call reports beside them: the status word, to
+// page-locked memory, and a clock.
 __global__ void gather_arrays_kernel(BoundaryArrays a, const int64_t* __restrict__ slot_of, int64_t nv,
                                      const int* status, int* status_out, float4 clock, float* clock_out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -778,7 +779,8 @@ static cudaError_t spread_second_wave(const void* kernel, int threads, size_t sm
     if (e != cudaSuccess) return e;
     *alone = 116 * 1024;  // more than half of an SM's 227 KB
     *spread = groups > *resident + sms / 4 && groups <= *resident + sms;
-    return *spread ? cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*alone) : cudaSuccess;
+    if (!*spread) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*alone);
 }
 
 // The colour2 step of groups of tiles with 4 slots a lane and no register cap, in scalar instructions (the results
@@ -792,11 +794,13 @@ static cudaError_t launch_scalar_groups(const DeviceState& st, const PhysParams&
     int64_t resident = 0;
     size_t alone = 0;
     bool spread = false;
-    cudaError_t e = spread_second_wave((const void*)scalar_group_kernel<4>, threads, 0, groups, &resident, &alone, &spread);
+    cudaError_t e =
+        spread_second_wave((const void*)scalar_group_kernel<4>, threads, 0, groups, &resident, &alone, &spread);
     if (e != cudaSuccess) return e;
     const unsigned first = spread ? (unsigned)resident : groups;
     scalar_group_kernel<4><<<first, threads, 0, s>>>(st, pp, sp, sdf, d_steps, nsteps, 0);
-    if (spread) scalar_group_kernel<4><<<groups - first, threads, alone, s>>>(st, pp, sp, sdf, d_steps, nsteps, (int)first);
+    if (spread)
+        scalar_group_kernel<4><<<groups - first, threads, alone, s>>>(st, pp, sp, sdf, d_steps, nsteps, (int)first);
     return cudaGetLastError();
 }
 
@@ -855,9 +859,9 @@ cudaError_t launch_fused_frame(const DeviceState& st, const PhysParams& pp, cons
 }
 
 template <typename K>
-static cudaError_t launch_persistent(K kernel, int64_t units, int threads, size_t smem, cudaStream_t s, const DeviceState& st,
-                                     const PhysParams& pp, const StepParams& sp, const SdfParams& sdf,
-                                     const StepParams* d_steps, int nsteps) {
+static cudaError_t launch_persistent(K kernel, int64_t units, int threads, size_t smem, cudaStream_t s,
+                                     const DeviceState& st, const PhysParams& pp, const StepParams& sp,
+                                     const SdfParams& sdf, const StepParams* d_steps, int nsteps) {
     unsigned grid = 0;
     cudaError_t e = persistent_grid((const void*)kernel, threads, smem, units, &grid);
     if (e != cudaSuccess) return e;
@@ -874,9 +878,11 @@ static cudaError_t launch_fused_persistent(const DeviceState& st, const PhysPara
     const int64_t units = (st.num_tiles + W - 1) / W;
     if (units == 0) return cudaSuccess;
     const int threads = 32 * W;
-#define KAMI_PERSIST(KERNEL, CC)                                                                                 \
-    return jacobi ? launch_persistent(KERNEL<CC, true>, units, threads, park_bytes(CC, W), s, st, pp, sp, sdf, d_steps, nsteps) \
-                  : launch_persistent(KERNEL<CC, false>, units, threads, park_bytes(CC, W), s, st, pp, sp, sdf, d_steps, nsteps)
+#define KAMI_PERSIST(KERNEL, CC)                                                                             \
+    return jacobi ? launch_persistent(KERNEL<CC, true>, units, threads, park_bytes(CC, W), s, st, pp, sp,    \
+                                      sdf, d_steps, nsteps)                                                  \
+                  : launch_persistent(KERNEL<CC, false>, units, threads, park_bytes(CC, W), s, st, pp, sp,   \
+                                      sdf, d_steps, nsteps)
     if (group > 1) {
         if (group > 8 || st.num_tiles % group != 0) return cudaErrorInvalidValue;
         if (C == 4 && !jacobi && reg_cap != 168)  // (launch_scalar_groups)
@@ -933,30 +939,27 @@ cudaError_t launch_fused_step(const DeviceState& st, const PhysParams& pp, const
     int threads = 32 * warps_per_block;
     unsigned blocks = blocks_for(st.num_tiles, warps_per_block);
     if (blocks == 0) return cudaSuccess;
+    const size_t park = park_bytes(C, warps_per_block);
     if (reg_cap == 168 && C == 4) {
         if (jacobi)
-            fused_step_kernel_r168<4, true><<<blocks, threads, park_bytes(4, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
-                nsteps);
+            fused_step_kernel_r168<4, true><<<blocks, threads, park, s>>>(st, pp, sp, sdf, d_steps, nsteps);
         else
-            fused_step_kernel_r168<4, false><<<blocks, threads, park_bytes(4, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
-                nsteps);
+            fused_step_kernel_r168<4, false><<<blocks, threads, park, s>>>(st, pp, sp, sdf, d_steps, nsteps);
         return cudaGetLastError();
     }
     if (reg_cap == 120 && C == 2) {
         if (jacobi)
-            fused_step_kernel_r120<2, true><<<blocks, threads, park_bytes(2, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
-                nsteps);
+            fused_step_kernel_r120<2, true><<<blocks, threads, park, s>>>(st, pp, sp, sdf, d_steps, nsteps);
         else
-            fused_step_kernel_r120<2, false><<<blocks, threads, park_bytes(2, warps_per_block), s>>>(st, pp, sp, sdf, d_steps,
-                nsteps);
+            fused_step_kernel_r120<2, false><<<blocks, threads, park, s>>>(st, pp, sp, sdf, d_steps, nsteps);
         return cudaGetLastError();
     }
 #define KAMI_FUSED_CASE(CC)                                                                        \
     if (C == CC) {                                                                                 \
         if (jacobi)                                                                                \
-            fused_step_kernel<CC, true><<<blocks, threads, park_bytes(CC, warps_per_block), s>>>(st, pp, sp, sdf, d_steps, nsteps);  \
+            fused_step_kernel<CC, true><<<blocks, threads, park, s>>>(st, pp, sp, sdf, d_steps, nsteps);  \
         else                                                                                       \
-            fused_step_kernel<CC, false><<<blocks, threads, park_bytes(CC, warps_per_block), s>>>(st, pp, sp, sdf, d_steps, nsteps); \
+            fused_step_kernel<CC, false><<<blocks, threads, park, s>>>(st, pp, sp, sdf, d_steps, nsteps); \
         return cudaGetLastError();                                                                 \
     }
     KAMI_FUSED_CASE(2)
