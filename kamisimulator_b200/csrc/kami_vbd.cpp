@@ -36,6 +36,7 @@ kami_status fail(kami_status st, const char* fmt, ...) {
 }
 
 kami_status cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();  // taken: the next call's launch check is not to find it
     if (e == cudaErrorMemoryAllocation) return fail(KAMI_ERR_OUT_OF_MEMORY, "%s: %s", what, cudaGetErrorString(e));
     return fail(KAMI_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }

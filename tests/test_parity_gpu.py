@@ -376,3 +376,20 @@ def test_exact_half_turns_count_as_not_positive(length, slots, schedule):
     finally:
         s.close()
     np.testing.assert_allclose(got, o.q, rtol=0, atol=1e-6)
+
+
+def test_a_refused_call_leaves_the_next_one_alone():
+    """A device pointer of another kind of memory is refused by the copy engine; the step after it runs."""
+    import ctypes
+
+    from kamisimulator_b200 import vbd
+
+    g = helpers.soft_groom(8, (8, 20), seed=5)
+    s = helpers.gpu_solver(g, helpers.soft_settings(num_itr=3))
+    try:
+        assert vbd.load_library().kami_vbd_get_state(s.handle, ctypes.c_void_p(16), ctypes.c_size_t(1 << 30),
+                                                     vbd.MEM_DEVICE) != vbd.KAMI_OK  # no memory there
+        s.step(1 / 60)
+        assert np.isfinite(s.get_positions_velocities()[0]).all()
+    finally:
+        s.close()
