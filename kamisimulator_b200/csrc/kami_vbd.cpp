@@ -332,16 +332,34 @@ kami_status stage_out(kami_vbd_solver* h, float* dst, int comps, int32_t memory)
     return KAMI_OK;
 }
 
-// Whether a kernel on the handle's device can read or write p itself: device memory of that device, or
-// managed memory.  Anything else goes through the staging buffer and the copy engine, as it always did.
-bool device_accessible(const kami_vbd_solver* h, const void* p) {
-    cudaPointerAttributes a{};
-    if (((uintptr_t)p & 3) != 0) return false;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return (a.type == cudaMemoryTypeDevice && a.device == h->device) || a.type == cudaMemoryTypeManaged;
+// Whether a kernel on the handle's device can read or write the n floats at p itself: device memory of that
+// device, or managed memory, and all of it in one allocation.  Anything else goes through the staging buffer and
+// the copy engine, as it always did, which refuses what is not there.
+bool device_accessible(const kami_vbd_solver* h, const void* p, int64_t n) {
+    using PtrAttrs = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const PtrAttrs ptr_attrs = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return (PtrAttrs) nullptr;
+        }
+        return (PtrAttrs)f;
+    }();
+    if (!ptr_attrs || !p || ((uintptr_t)p & 3) != 0) return false;
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                   CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0, managed = 0;
+    int device = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    void* out[5] = {&type, &device, &managed, &start, &size};
+    const CUdeviceptr d = (CUdeviceptr)(uintptr_t)p;
+    if (ptr_attrs(5, what, out, d) != CUDA_SUCCESS) return false;
+    if (!managed && !(type == CU_MEMORYTYPE_DEVICE && device == h->device)) return false;
+    return d >= start && d + sizeof(float) * (size_t)n <= start + size;
 }
 
 kami_status valid_handle(kami_vbd_solver* h) {
@@ -946,7 +964,8 @@ kami_status kami_vbd_get_sizes(kami_vbd_handle h, int64_t* num_vertices, int32_t
 kami_status kami_vbd_set_positions_velocities(kami_vbd_handle h, const float* xyz, const float* vxyz, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (memory != KAMI_MEMORY_HOST && memory != KAMI_MEMORY_DEVICE) return fail(KAMI_ERR_INVALID_ARGUMENT, "bad memory kind");
-    if (memory == KAMI_MEMORY_DEVICE && (!xyz || device_accessible(h, xyz)) && (!vxyz || device_accessible(h, vxyz))) {
+    if (memory == KAMI_MEMORY_DEVICE && (!xyz || device_accessible(h, xyz, 3 * h->nv)) &&
+        (!vxyz || device_accessible(h, vxyz, 3 * h->nv))) {
         BoundaryArrays a;
         if (xyz) a.add(h->d_xm, xyz, 3);
         if (vxyz) a.add(h->d_vel, vxyz, 3);
@@ -967,7 +986,8 @@ kami_status kami_vbd_set_positions_velocities(kami_vbd_handle h, const float* xy
 kami_status kami_vbd_get_positions_velocities(kami_vbd_handle h, float* xyz, float* vxyz, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (memory != KAMI_MEMORY_HOST && memory != KAMI_MEMORY_DEVICE) return fail(KAMI_ERR_INVALID_ARGUMENT, "bad memory kind");
-    if (memory == KAMI_MEMORY_DEVICE && (!xyz || device_accessible(h, xyz)) && (!vxyz || device_accessible(h, vxyz))) {
+    if (memory == KAMI_MEMORY_DEVICE && (!xyz || device_accessible(h, xyz, 3 * h->nv)) &&
+        (!vxyz || device_accessible(h, vxyz, 3 * h->nv))) {
         BoundaryArrays a;
         if (xyz) a.add(h->d_xm, xyz, 3);
         if (vxyz) a.add(h->d_vel, vxyz, 3);
@@ -991,7 +1011,7 @@ kami_status kami_vbd_get_positions_velocities(kami_vbd_handle h, float* xyz, flo
 static kami_status get4(kami_vbd_solver* h, const float4* src, float* dst, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (!dst) return fail(KAMI_ERR_INVALID_ARGUMENT, "null output");
-    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, dst)) {
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, dst, 4 * h->nv)) {
         BoundaryArrays a;
         a.add(const_cast<float4*>(src), dst, 4);
         KAMI_CUDA(launch_gather_arrays(a, h->d_slot_of, h->nv, nullptr, nullptr, float4{}, nullptr, h->stream), "gather");
@@ -1006,7 +1026,7 @@ static kami_status get4(kami_vbd_solver* h, const float4* src, float* dst, int32
 static kami_status set4(kami_vbd_solver* h, float4* dst, const float* src, int32_t memory) {
     KAMI_TRY(valid_handle(h));
     if (!src) return fail(KAMI_ERR_INVALID_ARGUMENT, "null input");
-    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, src)) {
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, src, 4 * h->nv)) {
         BoundaryArrays a;
         a.add(dst, src, 4);
         KAMI_CUDA(launch_scatter_arrays(a, h->d_slot_of, h->nv, h->stream), "scatter");
@@ -1721,8 +1741,9 @@ kami_status kami_vbd_backward(kami_vbd_handle h, float* adj_x, float* adj_v, flo
     const int64_t* wv = nullptr;
     int64_t ws0 = 0, wn = 0;
     if (memory == KAMI_MEMORY_DEVICE) KAMI_TRY(window_slots(h, &wv, &ws0, &wn));
-    const bool direct = memory == KAMI_MEMORY_DEVICE && device_accessible(h, adj_x) && device_accessible(h, adj_v) &&
-                        device_accessible(h, adj_vlast) && device_accessible(h, adj_q);
+    const bool direct = memory == KAMI_MEMORY_DEVICE && device_accessible(h, adj_x, 3 * h->nv) &&
+                        device_accessible(h, adj_v, 3 * h->nv) && device_accessible(h, adj_vlast, 3 * h->nv) &&
+                        device_accessible(h, adj_q, 4 * h->nv);
     if (wv) {
         for (int a = 0; a < 3; a++) {
             KAMI_CUDA(cudaMemsetAsync(adj3[a] + ws0, 0, sizeof(float4) * wn, h->stream), "adjoint reset");
@@ -1990,7 +2011,7 @@ kami_status kami_vbd_get_state(kami_vbd_handle h, void* dst, size_t bytes, int32
     float ctr_f;
     std::memcpy(&ctr_f, &ctr, 4);
     const float clk[4] = {h->h, h->last_h, h->time, ctr_f};
-    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, dst) && nv > 0) {
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, dst, 13 * nv + 4) && nv > 0) {
         BoundaryArrays a;
         a.add(h->d_xm, f, 3);
         a.add(h->d_vel, f + 3 * nv, 3);
@@ -2028,7 +2049,7 @@ kami_status kami_vbd_set_state(kami_vbd_handle h, const void* src, size_t bytes,
     cudaMemcpyKind kind = memory == KAMI_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     float4* dsts[3] = {h->d_xm, h->d_vel, h->d_vlast};
     float clk[4];
-    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, src)) {
+    if (memory == KAMI_MEMORY_DEVICE && device_accessible(h, src, 13 * nv + 4)) {
         BoundaryArrays a;
         for (int k = 0; k < 3; k++) a.add(dsts[k], f + 3 * nv * k, 3);
         a.add(h->d_q, f + 9 * nv, 4);

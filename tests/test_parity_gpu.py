@@ -379,17 +379,59 @@ def test_exact_half_turns_count_as_not_positive(length, slots, schedule):
 
 
 def test_a_refused_call_leaves_the_next_one_alone():
-    """A device pointer of another kind of memory is refused by the copy engine; the step after it runs."""
+    """A device array that ends too early is refused by the copy engine; the step after it runs."""
     import ctypes
 
     from kamisimulator_b200 import vbd
 
+    cu = ctypes.CDLL("libcuda.so.1")
     g = helpers.soft_groom(8, (8, 20), seed=5)
     s = helpers.gpu_solver(g, helpers.soft_settings(num_itr=3))
+    short = ctypes.c_uint64()
+    assert cu.cuMemAlloc_v2(ctypes.byref(short), ctypes.c_size_t(12 * s.num_vertices - 4)) == 0
     try:
-        assert vbd.load_library().kami_vbd_get_state(s.handle, ctypes.c_void_p(16), ctypes.c_size_t(1 << 30),
-                                                     vbd.MEM_DEVICE) != vbd.KAMI_OK  # no memory there
+        assert vbd.load_library().kami_vbd_get_positions_velocities(s.handle, ctypes.c_void_p(short.value), None,
+                                                                    vbd.MEM_DEVICE) != vbd.KAMI_OK
         s.step(1 / 60)
         assert np.isfinite(s.get_positions_velocities()[0]).all()
     finally:
         s.close()
+        cu.cuMemFree_v2(short)
+
+
+def test_device_arrays_that_end_too_early_are_refused():
+    """A device array that does not hold all the floats a call moves is left to the copy engine, which refuses it:
+    no kernel reads or writes past an allocation.  One of exactly the size is taken."""
+    import ctypes
+
+    from kamisimulator_b200 import vbd
+
+    cu = ctypes.CDLL("libcuda.so.1")
+    g = helpers.soft_groom(85, (50, 50), seed=5)
+    s = helpers.gpu_solver(g, helpers.soft_settings(num_itr=3), velocities=helpers.random_velocities(g))
+    nv, lib = s.num_vertices, vbd.load_library()
+
+    def alloc(nbytes):
+        p = ctypes.c_uint64()
+        assert cu.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t(nbytes)) == 0
+        return p.value
+
+    n = {"x": 12 * nv, "q": 16 * nv, "state": 4 * (13 * nv + 4)}
+    bufs = {k: (alloc(v), alloc(v - 4)) for k, v in n.items()}
+    h, p, dev = s.handle, ctypes.c_void_p, vbd.MEM_DEVICE
+    try:
+        for which, ok in ((0, True), (1, False)):
+            x, q, state = (p(bufs[k][which]) for k in ("x", "q", "state"))
+            for rc in (lib.kami_vbd_get_positions_velocities(h, x, None, dev),
+                       lib.kami_vbd_set_positions_velocities(h, x, None, dev),
+                       lib.kami_vbd_get_orientations(h, q, dev), lib.kami_vbd_set_orientations(h, q, dev),
+                       lib.kami_vbd_get_state(h, state, ctypes.c_size_t(n["state"]), dev),
+                       lib.kami_vbd_set_state(h, state, ctypes.c_size_t(n["state"]), dev)):
+                assert (rc == vbd.KAMI_OK) == ok
+        s.step(1 / 60)
+        assert np.isfinite(s.get_positions_velocities()[0]).all()
+    finally:
+        s.close()
+        for pair in bufs.values():
+            for b in pair:
+                cu.cuMemFree_v2(ctypes.c_uint64(b))
