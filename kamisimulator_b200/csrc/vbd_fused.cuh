@@ -150,12 +150,13 @@ __device__ __forceinline__ V3 half_axis(Q4 q) {
 }
 
 // A vertex's folded coefficients for one substep (see the file comment); zeros for a vertex that does not
-// move.  CHAINED: the order of the force's sum, which differs between the slots of a lane.
+// move.  The order of the force's sum differs between the slots of a lane.
+enum ForceOrder { CHAINED, HALF_CHAINED, SEPARATE };
 struct VertexFold {
     float3 F0;
     float as_, isA, isD;
 };
-template <bool CHAINED>
+template <ForceOrder ORDER>
 __device__ __forceinline__ VertexFold fold_vertex(float im, float h, float damp, float accel, float ddN, float ddP,
                                                   float3 y, float3 e, float3 eP) {
     const float a = im != 0.f ? 1.f / (im * h * h) : 0.f;
@@ -166,8 +167,8 @@ __device__ __forceinline__ VertexFold fold_vertex(float im, float h, float damp,
     b.isD = im != 0.f ? accel / fmaf(3.f, a, sk) - b.isA : 0.f;
     auto force = [&](float ya, float en, float ep) {
         const float n = __fmul_rn(ddN, en);  // a segment's product enters both its vertices
-        return CHAINED ? fmaf(-ddP, ep, fmaf(a, ya, n))
-                       : __fsub_rn(__fadd_rn(__fmul_rn(a, ya), n), __fmul_rn(ddP, ep));
+        if (ORDER == CHAINED) return fmaf(-ddP, ep, fmaf(a, ya, n));
+        return __fsub_rn(ORDER == HALF_CHAINED ? fmaf(a, ya, n) : __fadd_rn(__fmul_rn(a, ya), n), __fmul_rn(ddP, ep));
     };
     b.F0 = f3(force(y.x, e.x, eP.x), force(y.y, e.y, eP.y), force(y.z, e.z, eP.z));
     return b;
@@ -486,8 +487,8 @@ __device__ __forceinline__ void fused_step_body(DeviceState st, PhysParams pp, S
                 const float ddP = k > 0 ? ddN[k > 0 ? k - 1 : 0] : ddH;
                 const float3 eP = k > 0 ? e[k > 0 ? k - 1 : 0] : e0;
                 const VertexFold b = SHORT || k == 0 || (C == 2 && !HOSTIO)
-                                         ? fold_vertex<true>(im, h, damp, accel, ddN[k], ddP, y, e[k], eP)
-                                         : fold_vertex<false>(im, h, damp, accel, ddN[k], ddP, y, e[k], eP);
+                                         ? fold_vertex<CHAINED>(im, h, damp, accel, ddN[k], ddP, y, e[k], eP)
+                                         : fold_vertex<SEPARATE>(im, h, damp, accel, ddN[k], ddP, y, e[k], eP);
                 as_[k] = b.as_;
                 isA[k] = b.isA;
                 isD[k] = b.isD;

@@ -1,9 +1,12 @@
 // vbd_scalar.cuh -- the fused colour2 step (vbd_fused.cuh) in scalar FP32 instructions, state in registers: for
-// the recorded steps of the adjoint, and for few groups of tiles.
+// the recorded steps of the adjoint, and for groups of tiles.
 //
 // Every result equals the paired step's to the bit: each sum below is written with the operands, the order and
 // the contractions that the paired form takes for the same slot, so that a checkpoint, a recomputed segment, a
-// step, a host frame or several steps of one launch can follow one another in any mix.
+// step, a host frame or several steps of one launch can follow one another in any mix.  One case is left out: the
+// recorded step of single tiles with 4 slots a lane sums the force of slots 1 to 3 in an order of its own, which
+// its gradients have always had: another rounding of a step moves a stiffness gradient that sits on the kinks of
+// the predict's clamp or of the body pass by 1e-5 to 1e-4 of itself.  It is an ulp of the force away.
 //
 // What it is for.  A group's barriers make the chain of dependent instructions the bound, which the paired form's
 // moves between layouts lengthen (launch_scalar_groups has the times of both); and a recorded step is bound by the
@@ -230,9 +233,11 @@ __device__ __forceinline__ void scalar_step_body(DeviceState st, PhysParams pp, 
                 vl[k] = v[k];
                 const float ddP = k > 0 ? ddN[k > 0 ? k - 1 : 0] : ddH;
                 const float3 eP = k > 0 ? e[k > 0 ? k - 1 : 0] : eH;
-                const VertexFold b = SHORT || k == 0 || C == 2
-                                         ? fold_vertex<true>(im[k], h, damp, accel, ddN[k], ddP, y, e[k], eP)
-                                         : fold_vertex<false>(im[k], h, damp, accel, ddN[k], ddP, y, e[k], eP);
+                constexpr ForceOrder INNER = RECORD ? HALF_CHAINED : SEPARATE;  // of the slots 1 to 3 of 4
+                const bool chained = SHORT || k == 0 || C == 2 || (RECORD && k == C - 1);
+                const VertexFold b = chained
+                                         ? fold_vertex<CHAINED>(im[k], h, damp, accel, ddN[k], ddP, y, e[k], eP)
+                                         : fold_vertex<INNER>(im[k], h, damp, accel, ddN[k], ddP, y, e[k], eP);
                 as_[k] = b.as_;
                 isA[k] = b.isA;
                 isD[k] = b.isD;
