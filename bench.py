@@ -913,7 +913,8 @@ def run_ours(args):
                 "kernel_flop_per_vertex_iter": kernel_flop,
                 "achieved": per_gpu * kernel_flop / 1e12 if kernel_flop else None,
                 "issue_active": prof.get("issue_active_pct", 0) / 100 or None,
-                "source": "kernel FLOPs (2 FFMA + FMUL + FADD per thread) and issue-slot use from the committed ncu capture"}
+                "source": "kernel FLOPs (2 FFMA + FMUL + FADD per thread, counted on the step's scalar form; counters "
+                          "take a paired instruction once) and issue-slot use from the committed ncu capture"}
         fp32["frac"] = fp32["achieved"] / fp32_peak if fp32["achieved"] else None
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
