@@ -81,7 +81,8 @@ __device__ __forceinline__ OrientationAdjoint orientation_adjoint(float4 qbar, f
     s2 = nxt ? s2 : 0.f;
     const float4 b = make_float4(s1 * P1.x + s2 * P2.x, s1 * P1.y + s2 * P2.y, s1 * P1.z + s2 * P2.z,
                                  s1 * P1.w + s2 * P2.w);
-    // |V|, |b| and 1 / |R| as fused_orientation takes them (rsqrt forms), with the reciprocals the
+    // |V|, |b| and 1 / |R| as the step takes them (rsqrt forms; on groups of tiles it takes the lengths by
+    // sqrt.approx, an ulp or two away), with the reciprocals the
     // reverse needs: 1 / |V| = iV and 1 / |b| = ib wherever the norm is above 1e-15
     const float vv = dot3(V, V), bb2 = dot4(b, b);
     const float iV = rsqrt_ftz(fmaxf(vv, 1e-30f)), ib = rsqrt_ftz(fmaxf(bb2, 1e-30f));

@@ -781,8 +781,10 @@ static cudaError_t spread_second_wave(const void* kernel, int threads, size_t sm
     const int64_t rest = groups - *resident, per_sm = (rest + sms - 1) / sms;
     *spread = rest > sms / 4 && per_sm < *resident / sms && per_sm < 9;
     if (!*spread) return cudaSuccess;
-    *alone = (size_t)(204 * 1024 / per_sm);  // of 227 KB: per_sm CTAs fit, one more does not
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*alone);
+    constexpr int MOST = 204 * 1024;  // of 227 KB
+    *alone = (size_t)(MOST / per_sm);  // per_sm CTAs fit, one more does not
+    // (one limit for all: another thread may be launching the kernel with another share)
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
 }
 
 // The colour2 step of groups of tiles with 4 slots a lane and no register cap, in scalar instructions (the results

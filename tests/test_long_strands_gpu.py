@@ -244,3 +244,41 @@ def test_unpinned_long_strands_match_the_oracle(strands, slots):
     assert np.abs(x - o.x).max() <= helpers.POS_TOL
     assert np.abs(twist_angles(o.q, q)).max() <= helpers.TWIST_TOL
     np.testing.assert_array_equal(recorded, plain)
+
+
+def test_second_waves_of_two_handles_in_two_threads():
+    """Two handles whose second waves are spread to one and to two CTAs an SM, stepped from two threads at once:
+    the launches need different shares of shared memory and do not disturb one another."""
+    import threading
+
+    steps, out = 40, {}
+    st = _settings(num_itr=2)
+
+    def run(strands, key):
+        g = synth.groom_strands(np.random.default_rng(9), np.full(strands, 200))
+        s = helpers.gpu_solver(g, st, form="fused")
+        try:
+            assert s.tiles_per_group() == 2
+            barrier.wait()
+            for _ in range(steps):
+                s.step(1 / 120)
+            s.synchronize()
+            out[key] = s.get_state()
+        except Exception as exc:  # noqa: BLE001 - shown by the main thread
+            out[key] = exc
+        finally:
+            s.close()
+
+    for key in ("together", "apart"):
+        barrier = threading.Barrier(2 if key == "together" else 1)
+        threads = [threading.Thread(target=run, args=(n, (key, n))) for n in (660, 800)]
+        for t in threads:
+            t.start()
+            if key == "apart":
+                t.join()
+        for t in threads:
+            t.join()
+    for n in (660, 800):
+        for key in ("together", "apart"):
+            assert not isinstance(out[key, n], Exception), out[key, n]
+        np.testing.assert_array_equal(out["together", n], out["apart", n])
