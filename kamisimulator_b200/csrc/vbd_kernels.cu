@@ -164,9 +164,10 @@ __global__ void sweep_orientation_kernel(DeviceState st, const float4* __restric
 // the state is read once per iteration instead of once per sweep.  dx goes to dx_out, q is updated
 // in place.
 // Bound by latency: a launch, the loads, four dependent sweeps, the stores.  Launches are chained (grid_wait):
-// the tile's constants (positions, parameters, rest Darboux) are loaded while the launch before still runs.
-// A substep's first iteration is an ordinary launch, since the finish of the substep before wrote the positions.
-// 256,000 vertices, 20 iterations, the whole tied step: 211 us with ordinary launches, 190.
+// the tile's constants (parameters, rest Darboux) are loaded while the launch before still runs.  Positions are
+// read behind the wait: the finish of the substep before wrote them.  256,000 vertices, 20 iterations, the whole
+// tied step: 211 us with ordinary launches, 191 (190 with positions loaded early and an ordinary launch for a
+// substep's first iteration, but 1,200 vertices 63.8 us then and 62.0 so).
 __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, const float4* y4, float4* q,
                                                               const float4* dx_in,
                                                               float4* __restrict__ dx_out,
@@ -185,7 +186,6 @@ __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, co
     for (int c = 0; c < 2; c++) {
         const int p = (row2 + c) * 32 + lane;  // storage offset in the tile
         const int64_t g = base + p;
-        sx[p] = st.xm[g];
         sprm[p] = st.prm[g];
         sqr[p] = st.qr[g];
     }
@@ -197,6 +197,7 @@ __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, co
     for (int c = 0; c < 2; c++) {
         const int p = (row2 + c) * 32 + lane;
         yown[c] = xyz(load_fresh(y4 + base + p));
+        sx[p] = load_fresh(st.xm + base + p);
         sdx[p] = load_fresh(dx_in + base + p);
         sq[p] = load_fresh(q + base + p);
     }
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(512) sweep_iteration_kernel(DeviceState st, co
                 constexpr float k_tie = 4e1f;  // cosserat.cu:125
                 const BlockConst bc = vbd_block_const_tied(xm.w, fl, sn.dd, sp.dd, h, damp, k_tie);
                 const float3 f0 = bc.a * (yown[c] - dx) -
-                                  k_tie * ((xyz(xm) - xyz(st.xm[tie])) + (dx - xyz(load_fresh(dx_in + tie))) + damp * dx);
+                                  k_tie * ((xyz(xm) - xyz(load_fresh(st.xm + tie))) + (dx - xyz(load_fresh(dx_in + tie))) + damp * dx);
                 nd = vbd_position_from(f0, dx, fl, bc, sn.e, sn.invl, sn.kk, sn.dd, sn.d3, dxn, sp.e, sp.invl, sp.kk,
                                        sp.dd, sp.d3, dxp, damp, pp.accel_ratio);
             } else {
@@ -305,7 +306,6 @@ __global__ void __launch_bounds__(512) sweep_iteration_jacobi_kernel(DeviceState
     for (int c = 0; c < 2; c++) {
         const int p = (row2 + c) * 32 + lane;
         const int64_t g = base + p;
-        sx[p] = st.xm[g];
         sprm[p] = st.prm[g];
         sqr[p] = st.qr[g];
     }
@@ -317,6 +317,7 @@ __global__ void __launch_bounds__(512) sweep_iteration_jacobi_kernel(DeviceState
     for (int c = 0; c < 2; c++) {
         const int p = (row2 + c) * 32 + lane;
         yown[c] = xyz(load_fresh(y4 + base + p));
+        sx[p] = load_fresh(st.xm + base + p);
         sdx[p] = load_fresh(dx_in + base + p);
         sq[p] = load_fresh(q_in + base + p);
     }
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(512) sweep_iteration_jacobi_kernel(DeviceState
                 constexpr float k_tie = 4e1f;  // cosserat.cu:125
                 const BlockConst bc = vbd_block_const_tied(xm.w, fl, sn.dd, sp.dd, h, damp, k_tie);
                 const float3 f0 = bc.a * (yown[c] - dx) -
-                                  k_tie * ((xyz(xm) - xyz(st.xm[tie])) + (dx - xyz(load_fresh(dx_in + tie))) + damp * dx);
+                                  k_tie * ((xyz(xm) - xyz(load_fresh(st.xm + tie))) + (dx - xyz(load_fresh(dx_in + tie))) + damp * dx);
                 nd = vbd_position_from(f0, dx, fl, bc, sn.e, sn.invl, sn.kk, sn.dd, sn.d3, dxn, sp.e, sp.invl, sp.kk,
                                        sp.dd, sp.d3, dxp, damp, pp.accel_ratio);
             } else {

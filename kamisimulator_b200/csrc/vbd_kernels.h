@@ -34,6 +34,7 @@ cudaError_t launch_sweep_position(const DeviceState& st, const float4* y4, const
 // One iteration (colour2: both position sweeps, both orientation sweeps; jacobi: the position and
 // the orientation sweep) in one launch, one block per tile of up to 1024 slots: reads dx_in, writes
 // dx_out; q in place for colour2 (q_in == q_out), into q_out for jacobi (sweep_iteration_supported).
+// chained: behind the substep's prediction or another of its iterations.
 bool sweep_iteration_supported(int C);
 cudaError_t launch_sweep_iteration(const DeviceState& st, const float4* y4, const float4* q_in, float4* q_out,
                                    const float4* dx_in, float4* dx_out, const StepParams* d_sp, const PhysParams& pp,

@@ -41,9 +41,9 @@ def test_one_launch_iteration_equals_the_sweep_launches(tied, schedule):
 @pytest.mark.parametrize("schedule", ["colour2", "jacobi"])
 @pytest.mark.parametrize("strands", [40, 4000])
 def test_chained_iterations_follow_the_positions_of_every_substep(strands, schedule):
-    """Iterations behind a substep's first overlap the launch ahead of them and load the positions early;
-    with 12 substeps the positions change under them 11 times (few warps an SM and a full GPU, the two sides
-    on which iterations are chained).  The per-sweep launches are ordinary ones, so the state is the same."""
+    """Iterations overlap the launch ahead of them and read the positions behind their wait; with 12 substeps the
+    positions change under them 11 times (few warps an SM and a full GPU, the two sides on which iterations are
+    chained).  The per-sweep launches are ordinary ones, so the state is the same."""
     g = synth.groom(strands, 60, seed=23)
     st = dict(num_itr=6, max_h=1 / 1440, gravity=(0.0, 0.0, -9.81), radius=40e-6, schedule=schedule)
     one = helpers.gpu_solver(g, dict(st, slots_per_lane=2), form="sweep")
